@@ -1110,9 +1110,9 @@ extern "C" int mb_probabilities(mb_state s, const int* qubits, int nq, double* o
   if (rc) return rc;
   cudaStream_t st = g_ctx.stream;
   const double tol = std::sqrt(2.220446049250313e-16);  // _probability_tolerance (probabilities.jl:16-21)
-  MB_CHECK_CUDA(cudaMemsetAsync(d_out, 0, bytes, st));
   MB_CHECK_CUDA(cudaMemsetAsync(g_ctx.flags, 0, sizeof(unsigned) * 2, st));
-  rc = launch_marginal(s->d, s->n, is_dm, s->batch, qubits, nq, d_out, g_ctx.flags, tol, st);
+  rc = launch_marginal(s->d, s->n, is_dm, s->batch, qubits, nq, d_out, g_ctx.flags, tol,
+                       reinterpret_cast<double*>(g_ctx.partials), 2 * g_ctx.partials_cap, st);
   unsigned flags[2] = {0, 0};
   if (!rc) {
     cudaMemcpyAsync(out, d_out, bytes, cudaMemcpyDeviceToHost, st);

@@ -64,8 +64,9 @@ int launch_obs_apply(const double2* in, double2* out, int64_t elems, int nsample
 // ---- readout -------------------------------------------------------------------------------
 // Marginal probabilities: out[b * 2^nq + r] = sum of p_i over i whose readout bits form r.
 // For density matrices p_i = Re rho_ii; |Im rho_ii| > tol raises flags[0].
-int launch_marginal(const double2* v, int n, int is_dm, int nsamples, const int* qubits, int nq,
-                    double* out, unsigned* flags, double tol, cudaStream_t st);
+// Every bin of `out` is written. scratch: scratch_cap doubles for the partial sums of split bins.
+int launch_marginal(const double2* v, int n, int is_dm, int nsamples, const int* qubits, int nq, double* out,
+                    unsigned* flags, double tol, double* scratch, int64_t scratch_cap, cudaStream_t st);
 
 // ---- parameter binding -------------------------------------------------------------------------
 // One bind record per parametric instruction; the kernel writes its ordered matrix (and the

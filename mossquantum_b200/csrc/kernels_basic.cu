@@ -11,6 +11,7 @@
 // One thread owns one block of 2^K amplitudes that share all non-gate bits; consecutive
 // threads own consecutive blocks, so the loads of a warp are coalesced double2 (16 B)
 // accesses whenever the gate bits are not the lowest ones.
+#include <algorithm>
 #include <cstdarg>
 
 #include "family.cuh"
@@ -330,68 +331,114 @@ __global__ void k_obs_scalar(const double2* __restrict__ in, double2* __restrict
     out[i] = first ? cmul(s, in[i]) : cfma(s, in[i], out[i]);
 }
 
+// Marginal probabilities without atomics. The five lowest address bits are the lanes of a warp
+// (32 consecutive amplitudes, 512 B); a work unit is one value of the readout bits above them
+// and one of `splits` parts of the sum over the other high bits, which its warp runs through
+// with a masked increment, each lane in a register. Only then are the lanes whose index differs
+// in unread bits added (shuffles) and the bins written, each by one lane: no contention however
+// few the bins, and the same sum on every run. With splits > 1 the units write partial
+// histograms that k_marginal_sum adds in order.
+// Bound: one read of the state (HBM, or L2 up to about 2^22 amplitudes). Ten of 22 qubits: 16 us
+// and 4 us for the sum, against 36 us with a shared-memory histogram and double atomics.
 struct Readout {
   int nq;
-  int q[30];
+  int nh;                 // readout bits above the lanes
+  int hpos[32], hbin[32]; // their address bits (ascending) and bins' bits
+  int lbin[5];            // bin bit of lane bit l, or -1
+  uint64_t inner;         // high address bits that are summed over
+  int ninner;
 };
 
-// Marginal histogram in shared memory (nq <= 12), merged into out with double atomics.
-__global__ void __launch_bounds__(kBlock) k_marginal_small(const double2* __restrict__ v, int n, int is_dm,
-                                                            Readout ro, double* out, unsigned* flags, double tol) {
-  extern __shared__ double hist[];
-  const int b = blockIdx.y;
-  const int M = 1 << ro.nq;
-  const int64_t dim = int64_t(1) << n;
-  const int64_t elems = is_dm ? dim * dim : dim;
-  const double2* vs = v + int64_t(b) * elems;
-  for (int r = threadIdx.x; r < M; r += blockDim.x) hist[r] = 0.0;
-  __syncthreads();
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < dim; i += int64_t(gridDim.x) * blockDim.x) {
-    double p;
-    if (is_dm) {
-      double2 x = vs[i + dim * i];
-      if (fabs(x.y) > tol) atomicOr(&flags[0], 1u);
-      if (x.x < -tol) atomicOr(&flags[1], 1u);
-      p = x.x;
-    } else {
-      double2 x = vs[i];
-      p = x.x * x.x + x.y * x.y;
-    }
-    int r = 0;
-    for (int j = 0; j < ro.nq; ++j) r |= int((i >> ro.q[j]) & 1) << j;
-    atomicAdd(&hist[r], p);
-  }
-  __syncthreads();
-  for (int r = threadIdx.x; r < M; r += blockDim.x)
-    if (hist[r] != 0.0) atomicAdd(&out[int64_t(b) * M + r], hist[r]);
+__device__ __forceinline__ uint64_t deposit_mask(uint64_t x, uint64_t mask) {
+  uint64_t r = 0;
+  for (uint64_t m = mask; m && x; m &= m - 1, x >>= 1)
+    if (x & 1) r |= m & (~m + 1);
+  return r;
 }
 
-__global__ void __launch_bounds__(kBlock) k_marginal_large(const double2* __restrict__ v, int n, int is_dm,
-                                                            Readout ro, double* out, unsigned* flags, double tol,
-                                                            int identity) {
-  const int b = blockIdx.y;
-  const int64_t M = int64_t(1) << ro.nq;
-  const int64_t dim = int64_t(1) << n;
-  const int64_t elems = is_dm ? dim * dim : dim;
-  const double2* vs = v + int64_t(b) * elems;
-  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < dim; i += int64_t(gridDim.x) * blockDim.x) {
-    double p;
-    if (is_dm) {
-      double2 x = vs[i + dim * i];
-      if (fabs(x.y) > tol) atomicOr(&flags[0], 1u);
-      if (x.x < -tol) atomicOr(&flags[1], 1u);
-      p = x.x;
-    } else {
-      double2 x = vs[i];
-      p = x.x * x.x + x.y * x.y;
+template <bool DM>
+__global__ void __launch_bounds__(kBlock) k_marginal(const double2* __restrict__ v, int n, const Readout ro, int splits,
+                                                      int nsamples, double* out, unsigned* flags, double tol) {
+  const int lane = threadIdx.x & 31;
+  const int64_t dim = int64_t(1) << n, elems = DM ? dim * dim : dim;
+  const int64_t stride = DM ? dim + 1 : 1;
+  const int64_t M = int64_t(1) << ro.nq, units = (int64_t(nsamples) * splits) << ro.nh;
+  const int64_t nwarps = int64_t(gridDim.x) * (kBlock / 32);
+  const int64_t per = (int64_t(1) << ro.ninner) / splits;   // both powers of two
+  unsigned bad = 0;
+  for (int64_t u = int64_t(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5); u < units; u += nwarps) {
+    const int64_t h = u & ((int64_t(1) << ro.nh) - 1);
+    const int64_t rest = u >> ro.nh;
+    const int s = int(rest % splits), b = int(rest / splits);
+    uint64_t base = uint64_t(lane), bin = 0;
+    for (int k = 0; k < ro.nh; ++k) {
+      const uint64_t bit = (uint64_t(h) >> k) & 1;
+      base |= bit << ro.hpos[k];
+      bin |= bit << ro.hbin[k];
     }
-    if (identity) {
-      out[int64_t(b) * M + i] = p;
-    } else {
-      int64_t r = 0;
-      for (int j = 0; j < ro.nq; ++j) r |= ((i >> ro.q[j]) & 1) << j;
-      atomicAdd(&out[int64_t(b) * M + r], p);
+    const double2* vs = v + int64_t(b) * elems;
+    double p = 0.0;
+    if (lane < dim) {
+      uint64_t x = deposit_mask(uint64_t(s) * per, ro.inner);
+      int64_t i = 0;
+      for (; i + 4 <= per; i += 4) {
+        double2 a[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          a[k] = vs[int64_t(base | x) * stride];
+          x = ((x | ~ro.inner) + 1) & ro.inner;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (DM) {
+            bad |= (fabs(a[k].y) > tol ? 1u : 0u) | (a[k].x < -tol ? 2u : 0u);
+            p += a[k].x;
+          } else {
+            p += a[k].x * a[k].x + a[k].y * a[k].y;
+          }
+        }
+      }
+      for (; i < per; ++i) {
+        const double2 a = vs[int64_t(base | x) * stride];
+        x = ((x | ~ro.inner) + 1) & ro.inner;
+        if (DM) {
+          bad |= (fabs(a.y) > tol ? 1u : 0u) | (a.x < -tol ? 2u : 0u);
+          p += a.x;
+        } else {
+          p += a.x * a.x + a.y * a.y;
+        }
+      }
     }
+    bool mine = lane < dim;
+#pragma unroll
+    for (int l = 0; l < 5; ++l) {
+      const uint64_t bit = (lane >> l) & 1;
+      if (ro.lbin[l] < 0) {
+        p += __shfl_xor_sync(0xffffffffu, p, 1 << l);
+        mine = mine && bit == 0;
+      } else {
+        bin |= bit << ro.lbin[l];
+      }
+    }
+    if (mine) out[(int64_t(s) * nsamples + b) * M + int64_t(bin)] = p;
+  }
+  if (DM && bad) {
+    if (bad & 1u) atomicOr(&flags[0], 1u);
+    if (bad & 2u) atomicOr(&flags[1], 1u);
+  }
+}
+
+__global__ void __launch_bounds__(kBlock) k_marginal_sum(const double* __restrict__ part, int splits, int64_t count,
+                                                          double* __restrict__ out) {
+  // one warp per bin: lanes over the splits, then a fixed butterfly
+  const int lane = threadIdx.x & 31;
+  for (int64_t i = int64_t(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5); i < count;
+       i += int64_t(gridDim.x) * (kBlock / 32)) {
+    double p = 0.0;
+    for (int s = lane; s < splits; s += 32) p += part[int64_t(s) * count + i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+    if (lane == 0) out[i] = p;
   }
 }
 
@@ -563,25 +610,43 @@ int launch_obs_apply(const double2* in, double2* out, int64_t elems, int nsample
 }
 
 int launch_marginal(const double2* v, int n, int is_dm, int nsamples, const int* qubits, int nq, double* out,
-                    unsigned* flags, double tol, cudaStream_t st) {
+                    unsigned* flags, double tol, double* scratch, int64_t scratch_cap, cudaStream_t st) {
   if (nsamples <= 0) return MB_OK;
   Readout ro{};
   ro.nq = nq;
-  bool identity = nq == n;
-  for (int j = 0; j < nq; ++j) {
-    ro.q[j] = qubits[j];
-    identity = identity && qubits[j] == j;
+  for (int l = 0; l < 5; ++l) ro.lbin[l] = -1;
+  uint64_t read = 0;
+  for (int j = 0; j < nq; ++j) read |= uint64_t(1) << qubits[j];
+  for (int q = 0; q < n; ++q) {
+    if (!((read >> q) & 1)) {
+      if (q >= 5) ro.inner |= uint64_t(1) << q, ++ro.ninner;
+      continue;
+    }
+    const int j = int(std::find(qubits, qubits + nq, q) - qubits);
+    if (q < 5) ro.lbin[q] = j;
+    else ro.hpos[ro.nh] = q, ro.hbin[ro.nh++] = j;
   }
-  const int64_t dim = int64_t(1) << n;
-  // A pure state is read whole and a density matrix only on its diagonal: 16 B per entry read.
-  ProfScope ps(nq <= 12 && !identity ? "k_marginal_small" : "k_marginal_large", 16.0 * double(dim) * nsamples, st);
-  if (nq <= 12 && !identity) {
-    size_t shm = sizeof(double) << nq;
-    k_marginal_small<<<sample_grid(dim, nsamples), kBlock, shm, st>>>(v, n, is_dm, ro, out, flags, tol);
-  } else {
-    k_marginal_large<<<sample_grid(dim, nsamples), kBlock, 0, st>>>(v, n, is_dm, ro, out, flags, tol, identity);
+  // Split the sums while the units leave warps idle (64 warps per SM wanted), a part keeps at
+  // least 16 terms per lane, and the partial histograms fit the scratch.
+  const int64_t count = (int64_t(1) << nq) * nsamples;
+  int splits = 1;
+  while ((int64_t(nsamples) * splits << ro.nh) < int64_t(148) * 64 && (int64_t(1) << ro.ninner) / splits >= 32 &&
+         int64_t(splits) * 2 * count <= scratch_cap)
+    splits *= 2;
+  const int64_t units = (int64_t(nsamples) * splits) << ro.nh;
+  const int grid = grid_for(units, kBlock / 32, int64_t(148) * 8);
+  double* dst = splits > 1 ? scratch : out;
+  {
+    // A pure state is read whole and a density matrix only on its diagonal: 16 B per entry read.
+    ProfScope ps("k_marginal", 16.0 * double(int64_t(1) << n) * nsamples, st);
+    if (is_dm) k_marginal<true><<<grid, kBlock, 0, st>>>(v, n, ro, splits, nsamples, dst, flags, tol);
+    else k_marginal<false><<<grid, kBlock, 0, st>>>(v, n, ro, splits, nsamples, dst, flags, tol);
   }
   MB_LAUNCHED();
+  if (splits > 1) {
+    k_marginal_sum<<<grid_for(count, kBlock / 32, int64_t(148) * 8), kBlock, 0, st>>>(scratch, splits, count, out);
+    MB_LAUNCHED();
+  }
   return MB_OK;
 }
 

@@ -65,9 +65,9 @@ extern "C" int mb_qubit_weights(mb_state s, int qubit, double* w) {
   int rc = dev_alloc((void**)&d, bytes);
   if (rc) return rc;
   cudaStream_t st = g_ctx.stream;
-  cudaMemsetAsync(d, 0, bytes, st);
   cudaMemsetAsync(g_ctx.flags, 0, sizeof(unsigned) * 2, st);
-  rc = launch_marginal(s->d, s->n, is_dm, s->batch, &qubit, 1, d, g_ctx.flags, std::sqrt(2.220446049250313e-16), st);
+  rc = launch_marginal(s->d, s->n, is_dm, s->batch, &qubit, 1, d, g_ctx.flags, std::sqrt(2.220446049250313e-16),
+                       reinterpret_cast<double*>(g_ctx.partials), 2 * g_ctx.partials_cap, st);
   if (!rc) {
     cudaMemcpyAsync(w, d, bytes, cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) {
