@@ -11,8 +11,8 @@
 // Circuits with channels run on density matrices throughout (a pure initial state is
 // promoted first, DensityMatrix(psi), execution/channels.jl:19); this gives the same
 // parameter gradient as promoting at the first channel.
-// Fused paths: pure states (one sample) and density matrices (samples with shared parameters)
-// run the reverse as dual-state passes (y and Δ tiles together, gradients accumulated in the
+// Batches of density matrices enter as their weighted sum (the loss is linear in them).
+// Fused paths: pure states (one sample) and density matrices run the reverse as dual-state passes (y and Δ tiles together, gradients accumulated in the
 // pass). On density matrices a single-qubit channel is reversed by S' on Δ and S^-1 on y (the
 // input is uncomputed instead of recomputed); segments keep the product of ||S^-1||_2 within
 // 100 and y is reset to the segment's checkpoint after each, which bounds the rounding error.
@@ -60,6 +60,18 @@ static int gate_gradient(mb_circuit c, const COp& op, const double2* y, const do
   if (rc) return rc;
   for (int j = 0; j < op.k; ++j) p.p[j] = op.pos[j] + n;
   return launch_cross_dense(delta, y, elems, nsamples, p, D, 0, MAT_TRANSPOSE, ws(), 0, ro, g_ctx.stream);
+}
+
+// Seed of a density-matrix reverse: the matrix of H (z H' applied to the identity,
+// expectation.jl:69-73), from its strings where it has few, else key by key.
+static int seed_density(mb_observable o, double2* delta, int n, size_t sbytes) {
+  bool done = false;
+  if (int rc = seed_dm_strings(o, delta, n, &done)) return rc;
+  if (done) return MB_OK;
+  Buf ident;
+  if (int rc = ident.alloc(sbytes)) return rc;
+  if (int rc = launch_identity_density(ident.p, n, 1, g_ctx.stream)) return rc;
+  return observable_apply(o, ident.p, delta, n, 1, 1);
 }
 
 // Reverse of one application of a unitary circuit c on one pure sample, as used by the serving
@@ -189,22 +201,22 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
     set_error("adjoint gradients need a Hermitian observable");
     return MB_EUNSUPPORTED;
   }
-  const int B = init->batch;
+  int B = init->batch;
   if (B < 1) {
     set_error("scalar batch objectives require at least one sample");
     return MB_EINVAL;
   }
   const bool init_dm = init->kind == MB_DENSITY || init->kind == MB_BATCH_DENSITY;
   const int is_dm = (init_dm || c->has_channel) ? 1 : 0;
+  const bool batched = init->kind >= MB_BATCH_PURE;
   const int n = c->n;
   const int64_t elems = is_dm ? (int64_t(1) << (2 * n)) : (int64_t(1) << n);
-  const size_t sbytes = sizeof(double2) * size_t(elems) * B;
   cudaStream_t st = g_ctx.stream;
   int rc;
   if ((rc = bind_circuit(c, theta, ntheta, 1))) return rc;
 
   // Sample weights (the reduction of BatchExpectationObjective, api/objectives.jl:229-244).
-  std::vector<double> w(B, init->kind >= MB_BATCH_PURE ? 1.0 / B : 1.0);
+  std::vector<double> w(B, batched ? 1.0 / B : 1.0);
   if (weights) {
     for (int b = 0; b < B; ++b) {
       if (!std::isfinite(weights[b])) {
@@ -214,6 +226,11 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
       w[b] = weights[b];
     }
   }
+  // The weighted loss sum_b w_b tr(H E(rho_b)) is linear in the samples and they share the
+  // parameters, so on density matrices (batches, and pure batches promoted by a channel) the
+  // weighted sum of the samples goes through the circuit once in their place.
+  const bool combine = is_dm && B > 1;
+  const size_t sbytes = sizeof(double2) * size_t(elems) * (combine ? 1 : B);
   Buf d_w, d_grad, y, delta;
   if ((rc = d_w.alloc(sizeof(double) * B)) || (rc = d_grad.alloc(sizeof(double) * std::max(1, c->nslots))) ||
       (rc = y.alloc(sbytes)) || (rc = delta.alloc(sbytes)))
@@ -221,7 +238,12 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
   MB_CHECK_CUDA(cudaMemcpyAsync(d_w.p, w.data(), sizeof(double) * B, cudaMemcpyHostToDevice, st));
   double* d_g = reinterpret_cast<double*>(d_grad.p);
   MB_CHECK_CUDA(cudaMemsetAsync(d_g, 0, sizeof(double) * std::max(1, c->nslots), st));
-  if (is_dm && !init_dm) {
+  if (combine) {
+    if ((rc = launch_weighted_density(init->d, !init_dm, reinterpret_cast<double*>(d_w.p), B, n, y.p, st))) return rc;
+    B = 1;
+    w.assign(1, 1.0);
+    MB_CHECK_CUDA(cudaMemcpyAsync(d_w.p, w.data(), sizeof(double), cudaMemcpyHostToDevice, st));
+  } else if (is_dm && !init_dm) {
     if ((rc = launch_to_density(init->d, y.p, n, B, st))) return rc;
   } else {
     MB_CHECK_CUDA(cudaMemcpyAsync(y.p, init->d, sbytes, cudaMemcpyDeviceToDevice, st));
@@ -283,11 +305,8 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
   // circuit has channels): dual-state passes that reverse single-qubit channels with their
   // inverses. Segments end at checkpoint_every and wherever the product of the channels'
   // ||S^-1||_2 would pass 100, so the rounding error of the uncomputed y stays bounded; y is
-  // reset to the segment's checkpoint after each reversed segment. Shared parameters with
-  // uniform sample weights (the gradient sums over the samples and is scaled once).
-  bool uniform_w = true;
-  for (int b = 1; b < B; ++b) uniform_w = uniform_w && w[b] == w[0];
-  if (is_dm && uniform_w && 2 * n >= 8 && nops_all > 0 && !(plain_env && atoi(plain_env))) {
+  // reset to the segment's checkpoint after each reversed segment.
+  if (is_dm && 2 * n >= 8 && nops_all > 0 && !(plain_env && atoi(plain_env))) {
     std::vector<int> cuts = {0};
     bool ok = true;
     double growth = 1.0;
@@ -332,14 +351,8 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
       if ((rc = expect_keys(o, &view))) return rc;
       std::vector<double2> r(B);
       MB_CHECK_CUDA(cudaMemcpyAsync(r.data(), g_ctx.results, sizeof(double2) * B, cudaMemcpyDeviceToHost, st));
-      // seed: z H' applied to the identity, the dense matrix H per sample (expectation.jl:69-73)
-      {
-        Buf ident;
-        if ((rc = ident.alloc(sbytes))) return rc;
-        if ((rc = launch_identity_density(ident.p, n, B, st))) return rc;
-        if ((rc = observable_apply(o, ident.p, delta.p, n, 1, B))) return rc;
-        MB_CHECK_CUDA(cudaStreamSynchronize(st));
-      }
+      if ((rc = seed_density(o, delta.p, n, sbytes))) return rc;
+      MB_CHECK_CUDA(cudaStreamSynchronize(st));
       double v = 0;
       for (int b = 0; b < B; ++b) v += w[b] * r[b].x;
       *value = v;
@@ -399,12 +412,7 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
     if ((rc = observable_apply(o, y.p, delta.p, n, 0, B))) return rc;
     if ((rc = launch_scale(delta.p, elems * B, 2.0, st))) return rc;
   } else {
-    // z H' applied to the identity: the dense matrix H per sample.
-    Buf ident;
-    if ((rc = ident.alloc(sbytes))) return rc;
-    if ((rc = launch_identity_density(ident.p, n, B, st))) return rc;
-    if ((rc = observable_apply(o, ident.p, delta.p, n, 1, B))) return rc;
-    MB_CHECK_CUDA(cudaStreamSynchronize(st));
+    if ((rc = seed_density(o, delta.p, n, sbytes))) return rc;
   }
 
   // Reverse pass.

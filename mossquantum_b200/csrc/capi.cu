@@ -968,7 +968,10 @@ extern "C" int mb_observable_create(const mb_term* terms, size_t nterms, mb_obse
                                   g_ctx.stream));
     MB_CHECK_CUDA(cudaStreamSynchronize(g_ctx.stream));
   }
-  if (int rc = pauli_compile(o.get(), terms, nterms)) return rc;
+  if (int rc = pauli_compile(o.get(), terms, nterms)) {
+    dev_free(o->d_mats);
+    return rc;
+  }
   *out = o.release();
   return MB_OK;
 }
@@ -991,6 +994,11 @@ int expect_keys(mb_observable o, mb_state s, double2* out) {
   const int is_dm = s->kind == MB_DENSITY || s->kind == MB_BATCH_DENSITY;
   cudaStream_t st = g_ctx.stream;
   if (!out) out = g_ctx.results;
+  if (is_dm) {
+    bool done = false;
+    if (int rc = expect_dm_strings(o, s, out, &done)) return rc;
+    if (done) return MB_OK;
+  }
   MB_CHECK_CUDA(cudaMemsetAsync(out, 0, sizeof(double2) * s->batch, st));
   for (const OKey& k : o->keys) {
     ReduceOut ro{out, nullptr, nullptr, 1};

@@ -157,6 +157,10 @@ int expect_pauli(mb_observable o, mb_state s, double2* out = nullptr);
 // Whether Pauli programs built on the calling thread may compile specialised kernels (default
 // yes); when not, they run on the interpreter kernel.
 void pauli_allow_compile(bool on);
+// Density matrices: <H> per sample, or the matrix of H, from the observable's strings in one launch;
+// *done = false when the observable stays on its dense keys.
+int expect_dm_strings(mb_observable o, mb_state s, double2* out, bool* done);
+int seed_dm_strings(mb_observable o, double2* h, int n, bool* done);
 int pauli_apply(mb_observable o, const double2* in, double2* out, int n, int nsamples, double scale, bool* done);
 
 }  // namespace mb

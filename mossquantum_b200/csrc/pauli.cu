@@ -79,10 +79,19 @@ struct PauliProgram {
   double2* d_coef = nullptr;     // the observable's string coefficients, for the specialised kernels
 };
 
+// One flip mask of the observable: strings [s0, s0 + ns).
+struct PFlip {
+  uint64_t x;
+  int s0, ns;
+};
+
 struct PauliData {
   std::vector<PString> strings;  // grouped by flip mask
   std::vector<std::pair<uint64_t, std::pair<int, int>>> groups;  // x -> [s0, ns)
   std::vector<PauliProgram*> programs;
+  PFlip* d_flips = nullptr;      // groups and strings on the device (density matrices)
+  PString* d_all = nullptr;
+  int64_t dense_rows = 0;        // sum over the site keys of their matrix dimension
 };
 
 namespace {
@@ -297,6 +306,78 @@ __global__ void __launch_bounds__(kPThreads) k_pauli_apply(const double2* __rest
   }
 }
 
+// ---- density matrices -------------------------------------------------------------------------
+// H has entries only at (j ^ x, j) for the flip masks x of its strings, with
+//   f_x(j) = sum of c (-1)^{|j & z|} over the group's strings,
+// so tr(H rho) = sum over groups and j of f_x(j) rho[j, j ^ x]: a launch reads 2^n entries per flip
+// mask where the per-key kernels took a launch per site key and read each entry 2^k times.
+// Item (group, j), j fastest; latency bound at these sizes (XXZ on 9 qubits: 4,608 items).
+__device__ __forceinline__ double2 flip_factor(const PFlip& g, const PString* __restrict__ strings, uint64_t j) {
+  double2 f = cz();
+  for (int s = g.s0; s < g.s0 + g.ns; ++s) {
+    const PString p = strings[s];
+    const bool odd = __popcll(j & p.z) & 1;
+    f.x += odd ? -p.c.x : p.c.x;
+    f.y += odd ? -p.c.y : p.c.y;
+  }
+  return f;
+}
+
+__global__ void __launch_bounds__(kPThreads) k_dm_pauli(const double2* __restrict__ rho, int n,
+                                                       const PFlip* __restrict__ flips, int nflips,
+                                                       const PString* __restrict__ strings, int G, double2* partials,
+                                                       unsigned* counters, double2* out) {
+  __shared__ double2 wp[kPThreads / 32];
+  __shared__ bool last;
+  const int b = blockIdx.x / G, blk = blockIdx.x - b * G;
+  const int64_t dim = int64_t(1) << n, items = dim * nflips;
+  const double2* r = rho + int64_t(b) * dim * dim;
+  double2 acc = cz();
+  for (int64_t i = int64_t(blk) * kPThreads + threadIdx.x; i < items; i += int64_t(G) * kPThreads) {
+    const PFlip g = flips[i >> n];
+    const uint64_t j = uint64_t(i) & (dim - 1);
+    acc = cfma(flip_factor(g, strings, j), r[j + dim * (j ^ g.x)], acc);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    acc.x += __shfl_down_sync(0xffffffffu, acc.x, o);
+    acc.y += __shfl_down_sync(0xffffffffu, acc.y, o);
+  }
+  if ((threadIdx.x & 31) == 0) wp[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double2 s = cz();
+    for (int w = 0; w < kPThreads / 32; ++w) s = cadd(s, wp[w]);
+    partials[int64_t(b) * G + blk] = s;
+    __threadfence();
+    last = atomicAdd(&counters[b], 1u) == unsigned(G - 1);
+  }
+  __syncthreads();
+  if (!last || threadIdx.x >= 32) return;
+  // one warp adds the blocks' partials: lanes stride over them, then a fixed butterfly
+  double2 s = cz();
+  for (int g = threadIdx.x; g < G; g += 32) s = cadd(s, __ldcg(&partials[int64_t(b) * G + g]));
+  for (int o = 16; o > 0; o >>= 1) {
+    s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+    s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+  }
+  if (threadIdx.x == 0) {
+    out[b] = s;
+    counters[b] = 0;
+  }
+}
+
+// The matrix of H itself (zeroed before): entry (j ^ x, j) = f_x(j).
+__global__ void __launch_bounds__(kPThreads) k_dm_pauli_seed(double2* __restrict__ h, int n,
+                                                            const PFlip* __restrict__ flips, int nflips,
+                                                            const PString* __restrict__ strings) {
+  const int64_t dim = int64_t(1) << n, items = dim * nflips;
+  for (int64_t i = int64_t(blockIdx.x) * kPThreads + threadIdx.x; i < items; i += int64_t(gridDim.x) * kPThreads) {
+    const PFlip g = flips[i >> n];
+    const uint64_t j = uint64_t(i) & (dim - 1);
+    h[(j ^ g.x) + dim * j] = flip_factor(g, strings, j);
+  }
+}
+
 // Pauli coefficients of a 2x2 matrix M = sum_P a_P P with a_P = tr(P M)/2 (P in I,X,Y,Z).
 void pauli_decompose(const double* m, cdd a[4]) {
   const cdd m00(m[0], m[1]), m10(m[2], m[3]), m01(m[4], m[5]), m11(m[6], m[7]);
@@ -354,11 +435,74 @@ int pauli_compile(mb_observable o, const mb_term* terms, size_t nterms) {
   }
   o->pauli = pd;
   o->pauli_ok = true;
+  for (const OKey& k : o->keys) pd->dense_rows += int64_t(1) << k.k;
+  if (pd->strings.empty()) return MB_OK;
+  std::vector<PFlip> fl;
+  for (const auto& g : pd->groups) fl.push_back(PFlip{g.first, g.second.first, g.second.second});
+  int rc;
+  if ((rc = dev_alloc((void**)&pd->d_flips, sizeof(PFlip) * fl.size())) ||
+      (rc = dev_alloc((void**)&pd->d_all, sizeof(PString) * pd->strings.size()))) {
+    pauli_free(o);
+    return rc;
+  }
+  MB_CHECK_CUDA(cudaMemcpyAsync(pd->d_flips, fl.data(), sizeof(PFlip) * fl.size(), cudaMemcpyHostToDevice, g_ctx.stream));
+  MB_CHECK_CUDA(cudaMemcpyAsync(pd->d_all, pd->strings.data(), sizeof(PString) * pd->strings.size(),
+                                cudaMemcpyHostToDevice, g_ctx.stream));
+  MB_CHECK_CUDA(cudaStreamSynchronize(g_ctx.stream));
+  return MB_OK;
+}
+
+// Whether density matrices of n qubits take the string kernels. A string costs a sign and an add
+// per row of H, a row of a dense key a complex product per column, so observables of few strings
+// per key row gain (every spin chain: 3 strings per 4 rows, one launch of 8 us instead of one per
+// key); products of general 2x2 matrices on many sites, with up to 4^k strings, stay on the
+// dense keys (MB_EXPECT_KEYS=1 keeps every observable there).
+static bool dm_strings(const PauliData* pd, int n) {
+  const char* keys = getenv("MB_EXPECT_KEYS");
+  if (keys && atoi(keys) != 0) return false;
+  if (!pd || pd->strings.empty() || int64_t(pd->strings.size()) > 4 * pd->dense_rows) return false;
+  for (const auto& g : pd->groups)
+    if ((g.first >> n) != 0) return false;
+  for (const PString& s : pd->strings)
+    if ((s.z >> n) != 0) return false;
+  return true;
+}
+
+int expect_dm_strings(mb_observable o, mb_state s, double2* out, bool* done) {
+  PauliData* pd = o->pauli;
+  *done = false;
+  if (!dm_strings(pd, s->n)) return MB_OK;
+  const int64_t items = (int64_t(1) << s->n) * int64_t(pd->groups.size());
+  // two items per thread, at most four blocks per SM over all samples
+  const int64_t want = std::max<int64_t>(1, std::min<int64_t>((items + 2 * kPThreads - 1) / (2 * kPThreads),
+                                                             (int64_t(g_ctx.sm_count) * 4 + s->batch - 1) / s->batch));
+  const int G = int(std::min<int64_t>(want, g_ctx.partials_cap / s->batch));
+  if (G < 1 || s->batch > g_ctx.ncounters) return MB_OK;
+  ProfScope ps("k_dm_pauli", 16.0 * double(items) * s->batch, g_ctx.stream);
+  k_dm_pauli<<<unsigned(G * s->batch), kPThreads, 0, g_ctx.stream>>>(s->d, s->n, pd->d_flips, int(pd->groups.size()),
+                                                                    pd->d_all, G, g_ctx.partials, g_ctx.counters, out);
+  MB_LAUNCHED();
+  *done = true;
+  return MB_OK;
+}
+
+int seed_dm_strings(mb_observable o, double2* h, int n, bool* done) {
+  PauliData* pd = o->pauli;
+  *done = false;
+  if (!dm_strings(pd, n)) return MB_OK;
+  MB_CHECK_CUDA(cudaMemsetAsync(h, 0, sizeof(double2) << (2 * n), g_ctx.stream));
+  const int64_t items = (int64_t(1) << n) * int64_t(pd->groups.size());
+  k_dm_pauli_seed<<<grid_for(items, kPThreads), kPThreads, 0, g_ctx.stream>>>(h, n, pd->d_flips,
+                                                                             int(pd->groups.size()), pd->d_all);
+  MB_LAUNCHED();
+  *done = true;
   return MB_OK;
 }
 
 void pauli_free(mb_observable o) {
   if (!o->pauli) return;
+  dev_free(o->pauli->d_flips);
+  dev_free(o->pauli->d_all);
   for (PauliProgram* p : o->pauli->programs) {
     dev_free(p->d_groups);
     dev_free(p->d_strings);

@@ -457,9 +457,13 @@ void issue(mb_server S, size_t* res_off, int* nres) {
             if (!rc) rc = launch_scale(r->delta, c->elems, 2.0, st);
           }
         } else if (!rc) {
-          // delta = H as a density matrix (H applied to the identity)
-          rc = launch_identity_density(r->scratch[0], c->n, 1, st);
-          if (!rc) rc = observable_apply(r->obs, r->scratch[0], r->delta, c->n, 1, 1);
+          // delta = H as a density matrix (from its strings, or H applied to the identity)
+          bool seeded = false;
+          rc = seed_dm_strings(r->obs, r->delta, c->n, &seeded);
+          if (!rc && !seeded) {
+            rc = launch_identity_density(r->scratch[0], c->n, 1, st);
+            if (!rc) rc = observable_apply(r->obs, r->scratch[0], r->delta, c->n, 1, 1);
+          }
         }
         if (!rc) {
           r->phase = PH_REVERSE;
