@@ -249,6 +249,10 @@ MB_API int mb_observable_create(const mb_term* terms, size_t nterms, mb_observab
 MB_API int mb_observable_free(mb_observable o);
 /* <H> per sample: out holds 2 doubles (re, im) per sample (1 sample for single kinds). */
 MB_API int mb_expect(mb_observable o, mb_state s, double* out);
+/* <H> per sample after circuit c with parameters theta on a copy of init (a density matrix when
+ * c has channels); init is unchanged. Small pure states take one launch. out as for mb_expect. */
+MB_API int mb_objective_values(mb_circuit c, mb_observable o, mb_state init, const double* theta, size_t ntheta,
+                               double* out);
 /* out = H * in (execution/operators.jl:3-63); out has in's kind and shape. */
 MB_API int mb_observable_apply(mb_observable o, mb_state in, mb_state out);
 

@@ -132,6 +132,7 @@ def load():
         "mb_observable_create": ([ctypes.POINTER(MbTerm), sz, ctypes.POINTER(vp)], ctypes.c_int),
         "mb_observable_free": ([vp], ctypes.c_int),
         "mb_expect": ([vp, vp, dp], ctypes.c_int),
+        "mb_objective_values": ([vp, vp, vp, dp, sz, dp], ctypes.c_int),
         "mb_observable_apply": ([vp, vp, vp], ctypes.c_int),
         "mb_probabilities": ([vp, ip, ctypes.c_int, dp], ctypes.c_int),
         "mb_adjoint": ([vp, vp, vp, dp, sz, dp, ctypes.c_int, dp, dp], ctypes.c_int),

@@ -213,8 +213,7 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
   const int64_t elems = is_dm ? (int64_t(1) << (2 * n)) : (int64_t(1) << n);
   cudaStream_t st = g_ctx.stream;
   int rc;
-  if ((rc = bind_circuit(c, theta, ntheta, 1))) return rc;
-
+  if ((rc = theta_check(c, theta, ntheta, 1))) return rc;
   // Sample weights (the reduction of BatchExpectationObjective, api/objectives.jl:229-244).
   std::vector<double> w(B, batched ? 1.0 / B : 1.0);
   if (weights) {
@@ -226,6 +225,21 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
       w[b] = weights[b];
     }
   }
+  const char* plain_env = getenv("MB_ADJOINT_PLAIN");
+  const bool plain_only = plain_env && atoi(plain_env);
+  if (!is_dm && !plain_only) {
+    // small pure states: values and gradient in one launch
+    bool done = false;
+    std::vector<double2> v(B);
+    if ((rc = resident_run(c, o, init, theta, w.data(), v.data(), grad, &done))) return rc;
+    if (done) {
+      double total = 0;
+      for (int b = 0; b < B; ++b) total += w[b] * v[b].x;
+      *value = total;
+      return MB_OK;
+    }
+  }
+  if ((rc = bind_circuit(c, theta, ntheta, 1))) return rc;
   // The weighted loss sum_b w_b tr(H E(rho_b)) is linear in the samples and they share the
   // parameters, so on density matrices (batches, and pure batches promoted by a channel) the
   // weighted sum of the samples goes through the circuit once in their place.
@@ -251,8 +265,7 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
 
   // Fused path: pure single states with unitary circuits (specialised dual-state passes).
   const int nops_all = int(c->ops.size());
-  const char* plain_env = getenv("MB_ADJOINT_PLAIN");
-  if (!is_dm && B == 1 && !c->has_channel && n >= 9 && nops_all > 0 && !(plain_env && atoi(plain_env))) {
+  if (!is_dm && B == 1 && !c->has_channel && n >= 9 && nops_all > 0 && !plain_only) {
     const int kf = checkpoint_every > 0 ? checkpoint_every : nops_all;
     const int Sf = (nops_all + kf - 1) / kf;
     std::vector<Schedule*> adj(Sf, nullptr), fwd(Sf, nullptr);
@@ -306,7 +319,7 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
   // inverses. Segments end at checkpoint_every and wherever the product of the channels'
   // ||S^-1||_2 would pass 100, so the rounding error of the uncomputed y stays bounded; y is
   // reset to the segment's checkpoint after each reversed segment.
-  if (is_dm && 2 * n >= 8 && nops_all > 0 && !(plain_env && atoi(plain_env))) {
+  if (is_dm && 2 * n >= 8 && nops_all > 0 && !plain_only) {
     std::vector<int> cuts = {0};
     bool ok = true;
     double growth = 1.0;

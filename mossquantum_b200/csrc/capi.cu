@@ -113,6 +113,24 @@ static void norm_order(int k, const int* pos, int* sorted_pos, int* perm) {
   }
 }
 
+// Controlled single-target structure of a fixed ordered matrix: identity unless every
+// bit other than `tj` is 1. Returns the target local bit or -1.
+int controlled_target(const double2* M, int k) {
+  const int d = 1 << k;
+  for (int tj = 0; tj < k; ++tj) {
+    const int tb = 1 << tj, cm = (d - 1) & ~tb;
+    bool ok = true;
+    for (int r = 0; r < d && ok; ++r)
+      for (int c = 0; c < d && ok; ++c) {
+        const double2 x = M[r + c * d];
+        if ((r & ~tb) != (c & ~tb)) ok = (x.x == 0.0 && x.y == 0.0);
+        else if ((r & cm) != cm) ok = (r == c) ? (x.x == 1.0 && x.y == 0.0) : (x.x == 0.0 && x.y == 0.0);
+      }
+    if (ok) return tj;
+  }
+  return -1;
+}
+
 static int family_arity(int fam) {
   switch (fam) {
     case MB_FAM_RX: case MB_FAM_RY: case MB_FAM_RZ: case MB_FAM_PHASE: return 1;
@@ -201,6 +219,8 @@ extern "C" int mb_shutdown(void) {
   dev_free(g_ctx.counters);
   dev_free(g_ctx.results);
   dev_free(g_ctx.flags);
+  dev_free(g_ctx.d_small);
+  if (g_ctx.h_small) cudaFreeHost(g_ctx.h_small);
   cudaStreamSynchronize(g_ctx.stream);
   cudaStreamDestroy(g_ctx.stream);
   g_ctx = Ctx();
@@ -630,6 +650,7 @@ void circuit_release(mb_circuit c) {
     dev_free(c->d_binds);
     dev_free(c->d_theta);
     release_schedules(c);
+    resident_release(c);
   }
   if (c->h_theta) cudaFreeHost(c->h_theta);
   delete c;
@@ -696,9 +717,7 @@ int check_not_capturing(const char* what) {
   return MB_OK;
 }
 
-// Validates theta and stages it into the circuit's device parameter buffer (asynchronously,
-// through pinned memory); makes room for `rows` matrix-table rows.
-int theta_stage(mb_circuit c, const double* theta, size_t ntheta, int rows) {
+int theta_check(mb_circuit c, const double* theta, size_t ntheta, int rows) {
   if (ntheta != size_t(c->nslots) * rows) {
     set_error("expected %zu parameter values, got %zu", size_t(c->nslots) * rows, ntheta);
     return MB_EINVAL;
@@ -708,6 +727,33 @@ int theta_stage(mb_circuit c, const double* theta, size_t ntheta, int rows) {
       set_error("parameter values must be finite");
       return MB_EINVAL;
     }
+  return MB_OK;
+}
+
+int small_reserve(size_t host_doubles, size_t device_doubles) {
+  if (host_doubles + 2 > g_ctx.h_small_cap) {
+    const size_t cap = std::max<size_t>(2 * host_doubles, 4096);
+    double* p = nullptr;
+    MB_CHECK_CUDA(cudaMallocHost((void**)&p, sizeof(double) * cap));
+    if (g_ctx.h_small) cudaFreeHost(g_ctx.h_small);
+    g_ctx.h_small = p;
+    g_ctx.h_small_cap = cap;
+  }
+  if (device_doubles + 2 > g_ctx.d_small_cap) {
+    const size_t cap = std::max<size_t>(2 * device_doubles, 4096);
+    double* p = nullptr;
+    if (int rc = dev_alloc((void**)&p, sizeof(double) * cap)) return rc;
+    dev_free(g_ctx.d_small);
+    g_ctx.d_small = p;
+    g_ctx.d_small_cap = cap;
+  }
+  return MB_OK;
+}
+
+// Validates theta and stages it into the circuit's device parameter buffer (asynchronously,
+// through pinned memory); makes room for `rows` matrix-table rows.
+int theta_stage(mb_circuit c, const double* theta, size_t ntheta, int rows) {
+  if (int bad = theta_check(c, theta, ntheta, rows)) return bad;
   int rc;
   if (rows > c->table_rows) {
     double2* t = nullptr;
@@ -1048,6 +1094,52 @@ extern "C" int mb_expect(mb_observable o, mb_state s, double* out) {
   MB_CHECK_CUDA(cudaMemcpyAsync(out, g_ctx.results, sizeof(double2) * s->batch, cudaMemcpyDeviceToHost, g_ctx.stream));
   MB_CHECK_CUDA(cudaStreamSynchronize(g_ctx.stream));
   return MB_OK;
+}
+
+extern "C" int mb_objective_values(mb_circuit c, mb_observable o, mb_state init, const double* theta, size_t ntheta,
+                                   double* out) {
+  std::lock_guard<std::recursive_mutex> lk(g_mu);
+  if (int rc = check_init()) return rc;
+  if (int rc = check_not_capturing("mb_objective_values")) return rc;
+  if (!c || !o || !init || !out || (!theta && ntheta)) return MB_EINVAL;
+  if (init->n != c->n) {
+    set_error("circuit compiled for %d qubits, initial state has %d", c->n, init->n);
+    return MB_EINVAL;
+  }
+  if (int rc = validate_observable(o, init)) return rc;
+  if (int rc = theta_check(c, theta, ntheta, 1)) return rc;
+  if (init->batch == 0) return MB_OK;
+  if (init->batch > 65536) {
+    set_error("at most 65536 samples per expectation call");
+    return MB_EUNSUPPORTED;
+  }
+  bool done = false;
+  if (int rc = resident_run(c, o, init, theta, nullptr, reinterpret_cast<double2*>(out), nullptr, &done)) return rc;
+  if (done) return MB_OK;
+  // The general form: a private copy of the initial state through the fused passes.
+  const bool init_dm = init->kind == MB_DENSITY || init->kind == MB_BATCH_DENSITY;
+  const int kind = init_dm || !c->has_channel ? init->kind : init->kind == MB_PURE ? MB_DENSITY : MB_BATCH_DENSITY;
+  mb_state s = nullptr;
+  if (int rc = state_alloc(kind, init->n, init->batch, &s)) return rc;
+  int rc = MB_OK;
+  if (kind != init->kind) rc = launch_to_density(init->d, s->d, init->n, init->batch, g_ctx.stream);
+  else if (init->bytes && cudaMemcpyAsync(s->d, init->d, init->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream) != cudaSuccess) {
+    set_error("copy of the initial state failed: %s", cudaGetErrorString(cudaGetLastError()));
+    rc = MB_EDEVICE;
+  }
+  if (!rc) rc = bind_circuit(c, theta, ntheta, 1);
+  if (!rc) rc = apply_fused(c, s, 0);
+  if (!rc) rc = (o->pauli_ok && !init_dm && kind == init->kind) ? expect_pauli(o, s) : expect_keys(o, s);
+  if (!rc) {
+    cudaMemcpyAsync(out, g_ctx.results, sizeof(double2) * s->batch, cudaMemcpyDeviceToHost, g_ctx.stream);
+    const cudaError_t e = cudaStreamSynchronize(g_ctx.stream);
+    if (e != cudaSuccess) {
+      set_error("objective values: %s", cudaGetErrorString(e));
+      rc = MB_EDEVICE;
+    }
+  }
+  mb_state_free(s);
+  return rc;
 }
 
 namespace mb {

@@ -437,24 +437,6 @@ static double pass_flops_per_amp(const Pass& p, bool dual) {
 static bool is_one(double2 x) { return x.x == 1.0 && x.y == 0.0; }
 static bool is_zero(double2 x) { return x.x == 0.0 && x.y == 0.0; }
 
-// Controlled single-target structure of a fixed ordered matrix: identity unless every
-// bit other than `tj` is 1. Returns the target local bit or -1.
-static int controlled_target(const double2* M, int k) {
-  const int d = 1 << k;
-  for (int tj = 0; tj < k; ++tj) {
-    const int tb = 1 << tj, cm = (d - 1) & ~tb;
-    bool ok = true;
-    for (int r = 0; r < d && ok; ++r)
-      for (int c = 0; c < d && ok; ++c) {
-        const double2 x = M[r + c * d];
-        if ((r & ~tb) != (c & ~tb)) ok = is_zero(x);
-        else if ((r & cm) != cm) ok = (r == c) ? is_one(x) : is_zero(x);
-      }
-    if (ok) return tj;
-  }
-  return -1;
-}
-
 static void finalize_masks(FOp& f) {
   f.all = 0;
   for (int j = 0; j < f.nb; ++j) f.all |= uint64_t(1) << f.bits[j];

@@ -28,6 +28,7 @@ struct COp {
 };
 
 struct Schedule;       // fused-pass schedule (fused.cu)
+struct ResidentPlan;   // one-launch form for small pure states (resident.cu)
 
 struct mb_circuit_impl_tag {};
 
@@ -58,6 +59,7 @@ struct mb_circuit_s {
   size_t h_theta_cap = 0;
   int theta_rows = 0;                 // rows staged by the last theta upload
   std::vector<mb::Schedule*> scheds;  // fused schedules, built lazily per state shape
+  mb::ResidentPlan* resident = nullptr;  // built lazily by the first small objective
 };
 
 namespace mb {
@@ -67,6 +69,17 @@ struct OKey {
   int mat_off;
 };
 struct PauliData;    // pauli.cu
+
+// A Pauli string's Z mask and its coefficient, which includes i^{#Y}; the strings of one flip
+// mask x are [s0, s0 + ns) of the observable's array.
+struct PString {
+  uint64_t z;
+  double2 c;
+};
+struct PFlip {
+  uint64_t x;
+  int s0, ns;
+};
 }  // namespace mb
 
 struct mb_observable_s {
@@ -95,6 +108,9 @@ struct Ctx {
   int ncounters = 0;
   double2* results = nullptr;
   unsigned* flags = nullptr;
+  double* h_small = nullptr;        // small synchronous calls: pinned staging and its device side
+  double* d_small = nullptr;
+  size_t h_small_cap = 0, d_small_cap = 0;
   bool capturing = false;           // the library stream is recording a CUDA graph
   bool tensor_plain = false;        // per-gate path: dense 4-5 qubit ops on the tensor cores
 };
@@ -115,6 +131,12 @@ int state_alloc(int kind, int n, int batch, mb_state* out);
 int bind_circuit(mb_circuit c, const double* theta, size_t ntheta, int rows);
 int theta_stage(mb_circuit c, const double* theta, size_t ntheta, int rows);
 int bind_launch(mb_circuit c, int rows);
+int theta_check(mb_circuit c, const double* theta, size_t ntheta, int rows);
+// Room for so many doubles in h_small / d_small (and two more for alignment). Only for calls that
+// hold the library lock until their copies have finished.
+int small_reserve(size_t host_doubles, size_t device_doubles);
+// Target local bit of a fixed matrix that is the identity unless every other bit is 1, or -1.
+int controlled_target(const double2* M, int k);
 int check_not_capturing(const char* what);
 int plain_op(mb_circuit c, const COp& op, double2* v, int n, int is_dm, int nsamples, int64_t mrow_stride,
              bool dagger);
@@ -150,7 +172,21 @@ void dm_reverse_plan(mb_circuit c, int* seg_len, int* nscratch);
 int reverse_dm_single(mb_circuit c, int n, const double2* ckpt, double2* delta, double* d_grad,
                       double2* const* scratch);
 
+// resident.cu: small pure states, the whole objective in one launch. values: <H> per sample;
+// grad (or null): the gradient of the weighted sum. *done = false when the circuit, the
+// observable or the size has no resident form (nothing has been launched then).
+int resident_run(mb_circuit c, mb_observable o, mb_state init, const double* theta, const double* weights,
+                 double2* values, double* grad, bool* done);
+void resident_release(mb_circuit c);
+
 // pauli.cu
+// The observable's strings on the device; false when one acts outside n qubits.
+struct ObsStrings {
+  const PFlip* flips = nullptr;
+  const PString* strings = nullptr;
+  int nflips = 0, nstr = 0;
+};
+bool observable_strings(mb_observable o, int n, ObsStrings* out);
 int pauli_compile(mb_observable o, const mb_term* terms, size_t nterms);
 void pauli_free(mb_observable o);
 int expect_pauli(mb_observable o, mb_state s, double2* out = nullptr);

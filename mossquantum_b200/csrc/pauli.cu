@@ -40,11 +40,6 @@ template <int NR> struct PShape {
   static constexpr int per = tile / kPThreads;
 };
 
-struct PString {
-  uint64_t z;
-  double2 c;  // coefficient including i^{#Y}
-};
-
 // One flip-mask group of one pass; its strings are stored in the program's own order:
 // [k0, k0 + nk) constant per tile, [v0, v0 + nv) straddling, the rest tabulated at `tab`.
 struct PGroup {
@@ -77,12 +72,6 @@ struct PauliProgram {
   double2* d_tables = nullptr;
   std::vector<void*> jit;        // per pass: specialised expectation kernel (mbk_pauli) or null
   double2* d_coef = nullptr;     // the observable's string coefficients, for the specialised kernels
-};
-
-// One flip mask of the observable: strings [s0, s0 + ns).
-struct PFlip {
-  uint64_t x;
-  int s0, ns;
 };
 
 struct PauliData {
@@ -452,26 +441,34 @@ int pauli_compile(mb_observable o, const mb_term* terms, size_t nterms) {
   return MB_OK;
 }
 
+bool observable_strings(mb_observable o, int n, ObsStrings* out) {
+  const PauliData* pd = o->pauli;
+  if (!pd) return false;
+  for (const auto& g : pd->groups)
+    if ((g.first >> n) != 0) return false;
+  for (const PString& s : pd->strings)
+    if ((s.z >> n) != 0) return false;
+  *out = ObsStrings{pd->d_flips, pd->d_all, int(pd->groups.size()), int(pd->strings.size())};
+  return true;
+}
+
 // Whether density matrices of n qubits take the string kernels. A string costs a sign and an add
 // per row of H, a row of a dense key a complex product per column, so observables of few strings
 // per key row gain (every spin chain: 3 strings per 4 rows, one launch of 8 us instead of one per
 // key); products of general 2x2 matrices on many sites, with up to 4^k strings, stay on the
 // dense keys (MB_EXPECT_KEYS=1 keeps every observable there).
-static bool dm_strings(const PauliData* pd, int n) {
+static bool dm_strings(mb_observable o, int n) {
   const char* keys = getenv("MB_EXPECT_KEYS");
   if (keys && atoi(keys) != 0) return false;
-  if (!pd || pd->strings.empty() || int64_t(pd->strings.size()) > 4 * pd->dense_rows) return false;
-  for (const auto& g : pd->groups)
-    if ((g.first >> n) != 0) return false;
-  for (const PString& s : pd->strings)
-    if ((s.z >> n) != 0) return false;
-  return true;
+  const PauliData* pd = o->pauli;
+  ObsStrings os;
+  return observable_strings(o, n, &os) && os.nstr > 0 && int64_t(os.nstr) <= 4 * pd->dense_rows;
 }
 
 int expect_dm_strings(mb_observable o, mb_state s, double2* out, bool* done) {
   PauliData* pd = o->pauli;
   *done = false;
-  if (!dm_strings(pd, s->n)) return MB_OK;
+  if (!dm_strings(o, s->n)) return MB_OK;
   const int64_t items = (int64_t(1) << s->n) * int64_t(pd->groups.size());
   // two items per thread, at most four blocks per SM over all samples
   const int64_t want = std::max<int64_t>(1, std::min<int64_t>((items + 2 * kPThreads - 1) / (2 * kPThreads),
@@ -489,7 +486,7 @@ int expect_dm_strings(mb_observable o, mb_state s, double2* out, bool* done) {
 int seed_dm_strings(mb_observable o, double2* h, int n, bool* done) {
   PauliData* pd = o->pauli;
   *done = false;
-  if (!dm_strings(pd, n)) return MB_OK;
+  if (!dm_strings(o, n)) return MB_OK;
   MB_CHECK_CUDA(cudaMemsetAsync(h, 0, sizeof(double2) << (2 * n), g_ctx.stream));
   const int64_t items = (int64_t(1) << n) * int64_t(pd->groups.size());
   k_dm_pauli_seed<<<grid_for(items, kPThreads), kPThreads, 0, g_ctx.stream>>>(h, n, pd->d_flips,

@@ -11,7 +11,7 @@ from __future__ import annotations
 import numpy as np
 
 from . import _native as N
-from .backend import apply_, expectation
+from .backend import _validate_positions, backend, supports
 from .circuit import ParameterMap, QCircuit, accumulate_parameter_gradients
 from .operators import as_operator
 from .states import _DeviceState
@@ -59,8 +59,21 @@ class ExpectationObjective:
         return self.parameter_map.expand(values)
 
     def _sample_values(self, values):
-        state = apply_(self.template, self.initial_state.copy(), theta=self._slots(values))
-        return np.real(np.atleast_1d(expectation(self.observable, state)))
+        slots = self._slots(values)
+        template, state, op = self.template, self.initial_state, self.observable
+        if not supports(backend(state), template, state, "apply"):
+            raise N.UnsupportedOperation("B200Backend cannot apply this template")
+        _validate_positions(template, state.n)
+        if not supports(backend(state), op, state, "expectation"):
+            raise N.UnsupportedOperation("B200Backend cannot take the expectation of this observable")
+        if op.nqubits() > state.n:
+            raise ValueError("observable acts outside the register")
+        compiled = template.compiled(state.n)
+        theta = np.ascontiguousarray(compiled.theta_from(slots))
+        out = np.zeros(2 * state.batch)
+        N.check(N.lib().mb_objective_values(compiled.handle, op.handle().handle, state.handle, N.dptr(theta), theta.size,
+                                            N.dptr(out)), "evaluate")
+        return out[0::2].copy()
 
     def evaluate(self, values) -> float:
         return float(self._sample_values(values)[0])
