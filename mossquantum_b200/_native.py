@@ -128,14 +128,14 @@ def load():
                               ctypes.c_int, ip, ip, ip, ip, ip], ctypes.c_int),
         "mb_lowering_check": ([ctypes.POINTER(MbOp), sz, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                ctypes.c_uint64, dp, dp, dp], ctypes.c_int),
-        "mb_apply": ([vp, vp, dp, sz, ctypes.c_int], ctypes.c_int),
+        "mb_apply": ([vp, vp, vp, sz, ctypes.c_int], ctypes.c_int),
         "mb_observable_create": ([ctypes.POINTER(MbTerm), sz, ctypes.POINTER(vp)], ctypes.c_int),
         "mb_observable_free": ([vp], ctypes.c_int),
-        "mb_expect": ([vp, vp, dp], ctypes.c_int),
-        "mb_objective_values": ([vp, vp, vp, dp, sz, dp], ctypes.c_int),
+        "mb_expect": ([vp, vp, vp], ctypes.c_int),
+        "mb_objective_values": ([vp, vp, vp, vp, sz, vp], ctypes.c_int),
         "mb_observable_apply": ([vp, vp, vp], ctypes.c_int),
         "mb_probabilities": ([vp, ip, ctypes.c_int, dp], ctypes.c_int),
-        "mb_adjoint": ([vp, vp, vp, dp, sz, dp, ctypes.c_int, dp, dp], ctypes.c_int),
+        "mb_adjoint": ([vp, vp, vp, vp, sz, vp, ctypes.c_int, vp, vp], ctypes.c_int),
         "mb_theta_upload": ([vp, dp, sz, ctypes.c_int], ctypes.c_int),
         "mb_buffer_alloc": ([sz, ctypes.POINTER(vp)], ctypes.c_int),
         "mb_buffer_free": ([vp], ctypes.c_int),
@@ -260,6 +260,11 @@ def measure_fp64_peak() -> float:
 
 def synchronize() -> None:
     check(lib().mb_synchronize())
+
+
+def ptr(a: np.ndarray) -> int:
+    """Address of a contiguous array's data, for arguments declared as void pointers."""
+    return a.__array_interface__["data"][0]
 
 
 def dptr(a: np.ndarray):

@@ -53,7 +53,7 @@ def supports(b, operation, state, action="apply") -> bool:
         return False
     if action == "expectation":
         if isinstance(operation, (QubitsTerm, QubitsOperator)):
-            return all(len(t.positions) <= 5 for t in as_operator(operation).terms)
+            return as_operator(operation).facts()[2] <= 5
         return False
     if action == "probabilities":
         return True
@@ -102,21 +102,33 @@ def apply_(operation, state, theta=None, plain=False, tensor=False):
     if not isinstance(state, _DeviceState):
         raise TypeError("apply_ needs a B200 state")
     circuit = _as_circuit(operation) if isinstance(operation, (Gate, QCircuit)) else None
-    lowered = _matrix_lowering(circuit.flat()) if circuit is not None else None
-    if lowered is not None and _matrix_ops_fit(lowered[1], state.n):
-        # matrix and fixed gates of at most five qubits inside the register: supported, no
-        # channels, no parameters; the lowering doubles as the compile-cache signature
-        compiled = circuit.compiled(state.n, lowered=lowered)
-        values = np.zeros(0) if theta is None else theta
-    else:
-        if not supports(_BACKEND, operation, state, "apply"):
-            raise UnsupportedOperation(f"B200Backend cannot apply {type(operation).__name__}")
-        _validate_positions(operation, state.n)
-        circuit = _as_circuit(operation)
-        if circuit.has_channel() and not state.is_density:
+    key = circuit.value_key() if circuit is not None else None
+    known = circuit.known(state.n, key) if circuit is not None else None
+    if known is not None:
+        # these values passed the checks below on an earlier call
+        compiled, has_channel = known
+        if has_channel and not state.is_density:
             state = density_of(state)
-        compiled = circuit.compiled(state.n)
         values = circuit.active_parameters() if theta is None else theta
+    else:
+        lowered = _matrix_lowering(circuit.flat()) if circuit is not None else None
+        if lowered is not None and _matrix_ops_fit(lowered[1], state.n):
+            # matrix and fixed gates of at most five qubits inside the register: supported, no
+            # channels, no parameters; the lowering doubles as the compile-cache signature
+            compiled = circuit.compiled(state.n, lowered=lowered)
+            values = np.zeros(0) if theta is None else theta
+        else:
+            if not supports(_BACKEND, operation, state, "apply"):
+                raise UnsupportedOperation(f"B200Backend cannot apply {type(operation).__name__}")
+            _validate_positions(operation, state.n)
+            if circuit is None:
+                circuit = _as_circuit(operation)
+                key = circuit.value_key()
+            if circuit.has_channel() and not state.is_density:
+                state = density_of(state)
+            compiled = circuit.compiled(state.n, values=key)
+            values = circuit.active_parameters() if theta is None else theta
+        circuit.remember(state.n, compiled, key)
     values = np.asarray(values, dtype=np.float64)
     flags = N.MB_APPLY_PLAIN if plain else N.MB_APPLY_FUSED
     if plain and tensor:
@@ -126,7 +138,7 @@ def apply_(operation, state, theta=None, plain=False, tensor=False):
             raise ValueError("per-sample parameters need one row per batch sample")
         flags |= N.MB_APPLY_PER_SAMPLE
     th = np.ascontiguousarray(compiled.theta_from(values), dtype=np.float64)
-    N.check(N.lib().mb_apply(compiled.handle, state.handle, N.dptr(th), th.size, flags), "apply!")
+    N.check(N.lib().mb_apply(compiled.handle, state.handle, N.ptr(th), th.size, flags), "apply!")
     return state
 
 
@@ -140,12 +152,12 @@ def expectation(observable, state):
     if not supports(_BACKEND, observable, state, "expectation"):
         raise UnsupportedOperation(f"B200Backend cannot take the expectation of {type(observable).__name__}")
     op = as_operator(observable)
-    if op.nqubits() > state.n:
+    if op.facts()[1] > state.n:
         raise ValueError("observable acts outside the register")
     out = np.zeros(2 * max(state.batch, 1))
     if state.batch == 0:
         return np.zeros(0, dtype=complex)
-    N.check(N.lib().mb_expect(op.handle().handle, state.handle, N.dptr(out)), "expectation")
+    N.check(N.lib().mb_expect(op.handle().handle, state.handle, N.ptr(out)), "expectation")
     vals = out[0::2] + 1j * out[1::2]
     return vals if state.is_batch else complex(vals[0])
 

@@ -9,6 +9,7 @@ rebinding never recompiles the circuit.
 from __future__ import annotations
 
 import itertools
+import operator
 import weakref
 
 import numpy as np
@@ -23,9 +24,11 @@ class QCircuit(Instruction):
 
     def __init__(self, items=()):
         self.items = []
+        self._compiled = {}
+        self._known = {}     # register size -> (value key, (compiled circuit, has channels))
+        self._layout = None
         for it in items:
             self.push(it)
-        self._compiled = {}
 
     def push(self, item):
         from .measurement import QMeasure, QSelect
@@ -46,6 +49,7 @@ class QCircuit(Instruction):
         for handle in getattr(self, "_compiled", {}).values():
             handle.close()
         self._compiled = {}
+        self._known = {}
 
     def __iter__(self):
         return iter(self.items)
@@ -131,12 +135,18 @@ class QCircuit(Instruction):
         return [it.spec() for it in self.flat()]
 
     # lowering ---------------------------------------------------------------------------
-    def compiled(self, n: int, lowered=None) -> "CompiledCircuit":
+    def compiled(self, n: int, lowered=None, values=None) -> "CompiledCircuit":
         """The C-ABI circuit for an n-qubit register (cached; parameter values excluded).
-        lowered: this circuit's ``_matrix_lowering`` when the caller has it already."""
+        lowered, values: this circuit's ``_matrix_lowering`` and ``value_key`` when the caller has
+        them already."""
         if lowered is None:
             lowered = _matrix_lowering(self.flat())
-        key = (n, lowered[0] if lowered is not None else self._signature())
+        if lowered is not None:
+            key = (n, lowered[0])
+        else:
+            if values is None:
+                values = self.value_key()
+            key = (n, self._signature() if values is None else values)
         h = self._compiled.get(key)
         if h is None:
             if len(self._compiled) > 8:
@@ -144,6 +154,48 @@ class QCircuit(Instruction):
             h = CompiledCircuit(self, n, lowered)
             self._compiled[key] = h
         return h
+
+    def value_key(self):
+        """Everything that decides what this circuit compiles to and whether it may run, by value:
+        instruction types, positions, active flags, frozen parameter values, matrix and Kraus bytes
+        (values of active parameters are not part of it). None when an instruction is of a type
+        whose values this does not know. Read afresh on every call with C-level maps, an eighth of
+        the time of the per-instruction checks that it stands for."""
+        items = self.items
+        types = tuple(map(type, items))
+        if QCircuit in types:
+            items = self.flat()
+            types = tuple(map(type, items))
+        if self._layout is None or self._layout[0] != types:
+            kinds = [_item_kind(t) for t in types]
+            pick = [[i for i, k in enumerate(kinds) if k == want] for want in ("param", "map", "matrix")]
+            self._layout = (types, None not in kinds, *pick)
+        _, known, params, maps, mats = self._layout
+        if not known:
+            return None
+        pos = tuple(map(_get_pos, items))
+        if not set(map(type, pos)) <= {tuple}:
+            return None
+        try:
+            held = [items[i] for i in params]
+            active = tuple(map(tuple, map(_get_isparas, held)))
+            frozen = tuple([g.paras[0] for g, a in zip(held, active) if not a[0]])
+            kraus = list(map(_get_kraus, [items[i] for i in maps]))
+            return (types, pos, active, frozen, tuple(map(len, kraus)), b"".join(itertools.chain.from_iterable(kraus)),
+                    b"".join(map(_get_data, [items[i] for i in mats])))
+        except (AttributeError, BufferError, TypeError, ValueError, IndexError):
+            return None
+
+    def known(self, n, key):
+        """(compiled circuit, has channels) if ``remember`` was called for n and these values."""
+        kept = self._known.get(n)
+        return kept[1] if kept is not None and key is not None and kept[0] == key else None
+
+    def remember(self, n, compiled, key):
+        """Keep the compiled circuit of a program that passed every check on n qubits, under the
+        values (``value_key``) it was checked with."""
+        if key is not None:
+            self._known[n] = (key, (compiled, bool(self._layout[3])))
 
     def _signature(self):
         sig = []
@@ -169,6 +221,31 @@ class QCircuit(Instruction):
 
     def __repr__(self):
         return f"QCircuit({len(self.items)} instructions)"
+
+
+_get_pos = operator.attrgetter("pos")
+_get_isparas = operator.attrgetter("isparas")
+_get_kraus = operator.attrgetter("kraus")
+_get_data = operator.attrgetter("data")
+_item_kinds = {}
+
+
+def _item_kind(t):
+    """What a value key reads of an instruction of type t: "fixed" (type and positions), "param"
+    (one angle of a device family), "map" (Kraus matrices), "matrix" (its matrix), or None."""
+    if t not in _item_kinds:
+        from .gates import ParametricGate, QuantumGate, _FixedGate
+        kind = None
+        if issubclass(t, _FixedGate) and t._ops is _FixedGate._ops:
+            kind = "fixed"
+        elif issubclass(t, ParametricGate) and t._ops is ParametricGate._ops and t.family != "MATRIX":
+            kind = "param"
+        elif t is QuantumMap:
+            kind = "map"
+        elif t is QuantumGate:
+            kind = "matrix"
+        _item_kinds[t] = kind
+    return _item_kinds[t]
 
 
 _OP_DTYPE = np.dtype(N.MbOp)   # mb_op as a numpy record (same layout as the ctypes struct)
@@ -238,6 +315,7 @@ class CompiledCircuit:
             self.nslots = 0
             self.nparams = 0
             self.slot_map = []
+            self._slot_index()
             self.gradient_ok = True
             h = N.ctypes.c_void_p()
             arr = recs.ctypes.data_as(N.ctypes.POINTER(N.MbOp))
@@ -263,6 +341,7 @@ class CompiledCircuit:
         self.nslots = slot
         self.nparams = circuit.nparameters()
         self.slot_map = self._slot_map(circuit)
+        self._slot_index()
         self.gradient_ok = gradient_ok and self.nslots == self.nparams
         arr = (N.MbOp * max(1, len(ops)))(*ops)
         h = N.ctypes.c_void_p()
@@ -287,12 +366,27 @@ class CompiledCircuit:
                     out.append(-1)
         return out
 
+    def _slot_index(self):
+        """Parameters that reach the device, and whether they are all of them in order."""
+        self._in_slots = np.array([i for i, s in enumerate(self.slot_map) if s >= 0], dtype=np.intp)
+        self._slots = np.array([s for s in self.slot_map if s >= 0], dtype=np.intp)
+        self._plain_slots = self._in_slots.size == self.nparams and bool(np.all(self._slots == np.arange(self._slots.size)))
+
     def theta_from(self, values):
         values = np.asarray(values, dtype=np.float64)
         if values.shape[-1] != self.nparams:
             raise ValueError(f"expected {self.nparams} parameter values, got {values.shape[-1]}")
-        idx = [i for i, s in enumerate(self.slot_map) if s >= 0]
-        return np.ascontiguousarray(values[..., idx])
+        if self._in_slots.size == self.nparams:
+            return np.ascontiguousarray(values)
+        return np.ascontiguousarray(values[..., self._in_slots])
+
+    def gradient_from(self, slot_gradient):
+        """One entry per active parameter from the device's slots (0 where frozen into a matrix)."""
+        if self._plain_slots:
+            return slot_gradient[:self.nparams].copy()
+        out = np.zeros(self.nparams)
+        out[self._in_slots] = slot_gradient[self._slots]
+        return out
 
     def passes(self):
         v = N.ctypes.c_int()
@@ -327,6 +421,9 @@ class ParameterMap:
         if set(idx) != set(range(1, k + 1)):
             raise ValueError("parameter ids must cover 1:k without gaps")
         self._indices = tuple(idx)
+        self._count = k
+        self._index = np.array(idx, dtype=np.intp) - 1
+        self._one_to_one = idx == list(range(1, k + 1))
 
     def parameter_indices(self):
         return list(self._indices)
@@ -335,13 +432,13 @@ class ParameterMap:
         return len(self._indices)
 
     def nparameters(self):
-        return max(self._indices) if self._indices else 0
+        return self._count
 
     def expand(self, values):
         values = np.asarray(values, dtype=np.float64)
         if values.shape[-1] != self.nparameters():
             raise ValueError(f"expected {self.nparameters()} values, got {values.shape[-1]}")
-        return values[..., [i - 1 for i in self._indices]]
+        return values[..., self._index]
 
     def __eq__(self, other):
         return isinstance(other, ParameterMap) and other._indices == self._indices
@@ -355,6 +452,8 @@ def accumulate_parameter_gradients(parameter_map: ParameterMap, flat_gradient):
     g = np.asarray(flat_gradient, dtype=np.float64)
     if g.shape[-1] != len(parameter_map):
         raise ValueError("one gradient entry per slot required")
+    if parameter_map._one_to_one:
+        return g.copy()
     out = np.zeros(g.shape[:-1] + (parameter_map.nparameters(),))
     for i, j in enumerate(parameter_map.parameter_indices()):
         out[..., j - 1] += g[..., i]

@@ -221,6 +221,10 @@ extern "C" int mb_shutdown(void) {
   dev_free(g_ctx.flags);
   dev_free(g_ctx.d_small);
   if (g_ctx.h_small) cudaFreeHost(g_ctx.h_small);
+  for (auto& h : g_ctx.h_theta) {
+    if (h.p) cudaFreeHost(h.p);
+    if (h.copied) cudaEventDestroy(h.copied);
+  }
   cudaStreamSynchronize(g_ctx.stream);
   cudaStreamDestroy(g_ctx.stream);
   g_ctx = Ctx();
@@ -652,7 +656,6 @@ void circuit_release(mb_circuit c) {
     release_schedules(c);
     resident_release(c);
   }
-  if (c->h_theta) cudaFreeHost(c->h_theta);
   delete c;
 }
 
@@ -774,15 +777,26 @@ int theta_stage(mb_circuit c, const double* theta, size_t ntheta, int rows) {
     c->theta_cap = need;
   }
   if (ntheta) {
-    if (c->h_theta_cap < ntheta) {
-      if (c->h_theta) cudaFreeHost(c->h_theta);
-      MB_CHECK_CUDA(cudaMallocHost((void**)&c->h_theta, sizeof(double) * ntheta));
-      c->h_theta_cap = ntheta;
+    if (ntheta > kThetaStage) {
+      // pageable source: the copy has left it when the call returns
+      MB_CHECK_CUDA(cudaMemcpyAsync(c->d_theta, theta, sizeof(double) * ntheta, cudaMemcpyHostToDevice, g_ctx.stream));
+      return MB_OK;
     }
-    MB_CHECK_CUDA(cudaStreamSynchronize(g_ctx.stream));
-    std::memcpy(c->h_theta, theta, sizeof(double) * ntheta);
-    MB_CHECK_CUDA(cudaMemcpyAsync(c->d_theta, c->h_theta, sizeof(double) * ntheta, cudaMemcpyHostToDevice,
-                                  g_ctx.stream));
+    auto& h = g_ctx.h_theta[g_ctx.h_theta_next];
+    g_ctx.h_theta_next = (g_ctx.h_theta_next + 1) % 8;
+    if (!h.copied) MB_CHECK_CUDA(cudaEventCreateWithFlags(&h.copied, cudaEventDisableTiming));
+    else MB_CHECK_CUDA(cudaEventSynchronize(h.copied));
+    if (h.cap < ntheta) {
+      const size_t cap = std::max<size_t>(4096, 2 * ntheta);
+      if (h.p) cudaFreeHost(h.p);
+      h.p = nullptr;
+      h.cap = 0;
+      MB_CHECK_CUDA(cudaMallocHost((void**)&h.p, sizeof(double) * cap));
+      h.cap = cap;
+    }
+    std::memcpy(h.p, theta, sizeof(double) * ntheta);
+    MB_CHECK_CUDA(cudaMemcpyAsync(c->d_theta, h.p, sizeof(double) * ntheta, cudaMemcpyHostToDevice, g_ctx.stream));
+    MB_CHECK_CUDA(cudaEventRecord(h.copied, g_ctx.stream));
   }
   return MB_OK;
 }

@@ -55,8 +55,6 @@ struct mb_circuit_s {
   int table_rows = 1;
   double* d_theta = nullptr;
   size_t theta_cap = 0;
-  double* h_theta = nullptr;          // pinned staging for theta uploads
-  size_t h_theta_cap = 0;
   int theta_rows = 0;                 // rows staged by the last theta upload
   std::vector<mb::Schedule*> scheds;  // fused schedules, built lazily per state shape
   mb::ResidentPlan* resident = nullptr;  // built lazily by the first small objective
@@ -95,6 +93,8 @@ struct mb_observable_s {
 
 namespace mb {
 
+constexpr size_t kThetaStage = size_t(1) << 20;
+
 struct Ctx {
   bool init = false;
   int device = 0;
@@ -111,6 +111,15 @@ struct Ctx {
   double* h_small = nullptr;        // small synchronous calls: pinned staging and its device side
   double* d_small = nullptr;
   size_t h_small_cap = 0, d_small_cap = 0;
+  // Pinned staging for theta uploads of at most kThetaStage doubles, used in turn: a buffer is
+  // reused once its own copy has been made, so callers run ahead of the device instead of
+  // waiting for it. Larger uploads go from the caller's memory. Freed by mb_shutdown.
+  struct ThetaBuf {
+    double* p = nullptr;
+    size_t cap = 0;
+    cudaEvent_t copied = nullptr;
+  } h_theta[8];
+  int h_theta_next = 0;
   bool capturing = false;           // the library stream is recording a CUDA graph
   bool tensor_plain = false;        // per-gate path: dense 4-5 qubit ops on the tensor cores
 };

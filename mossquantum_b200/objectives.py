@@ -61,18 +61,24 @@ class ExpectationObjective:
     def _sample_values(self, values):
         slots = self._slots(values)
         template, state, op = self.template, self.initial_state, self.observable
-        if not supports(backend(state), template, state, "apply"):
-            raise N.UnsupportedOperation("B200Backend cannot apply this template")
-        _validate_positions(template, state.n)
+        key = template.value_key()
+        known = template.known(state.n, key)
+        if known is None:
+            if not supports(backend(state), template, state, "apply"):
+                raise N.UnsupportedOperation("B200Backend cannot apply this template")
+            _validate_positions(template, state.n)
+            compiled = template.compiled(state.n, values=key)
+            template.remember(state.n, compiled, key)
+        else:
+            compiled = known[0]
         if not supports(backend(state), op, state, "expectation"):
             raise N.UnsupportedOperation("B200Backend cannot take the expectation of this observable")
-        if op.nqubits() > state.n:
+        if op.facts()[1] > state.n:
             raise ValueError("observable acts outside the register")
-        compiled = template.compiled(state.n)
-        theta = np.ascontiguousarray(compiled.theta_from(slots))
+        theta = compiled.theta_from(slots)
         out = np.zeros(2 * state.batch)
-        N.check(N.lib().mb_objective_values(compiled.handle, op.handle().handle, state.handle, N.dptr(theta), theta.size,
-                                            N.dptr(out)), "evaluate")
+        N.check(N.lib().mb_objective_values(compiled.handle, op.handle().handle, state.handle, N.ptr(theta), theta.size,
+                                            N.ptr(out)), "evaluate")
         return out[0::2].copy()
 
     def evaluate(self, values) -> float:
@@ -126,13 +132,27 @@ def supports_gradient(method, objective) -> bool:
     from .sampled import SAMPLED_METHODS, supports_sampled
     if isinstance(method, SAMPLED_METHODS):
         return supports_sampled(method, objective)
+    return _gradient_circuit(method, objective) is not None
+
+
+def _gradient_circuit(method, objective):
+    """The compiled template if the adjoint method takes this objective, else None."""
     if not isinstance(method, AdjointGradient) or not isinstance(objective, ExpectationObjective):
-        return False
+        return None
+    template, n = objective.template, objective.initial_state.n
     try:
-        compiled = objective.template.compiled(objective.initial_state.n)
+        key = template.value_key()
+        known = template.known(n, key)
+        if known is not None:
+            compiled = known[0]
+        else:
+            compiled = template.compiled(n, values=key)
+            if supports(backend(objective.initial_state), template, objective.initial_state, "apply"):
+                _validate_positions(template, n)
+                template.remember(n, compiled, key)
     except Exception:
-        return False
-    return compiled.gradient_ok and objective.observable.is_hermitian()
+        return None
+    return compiled if compiled.gradient_ok and objective.observable.is_hermitian() else None
 
 
 def value_and_gradient(method, objective, values, rng=None):
@@ -143,27 +163,22 @@ def value_and_gradient(method, objective, values, rng=None):
     if isinstance(method, SAMPLED_METHODS):
         est = estimate_gradient(method, objective, values, rng=rng)
         return est.value, est.gradient
-    if not supports_gradient(method, objective):
+    compiled = _gradient_circuit(method, objective)
+    if compiled is None:
         raise UnsupportedGradient(f"{method!r} does not support this objective")
     slots = objective._slots(values)
     state = objective.initial_state
-    compiled = objective.template.compiled(state.n)
-    theta = np.ascontiguousarray(compiled.theta_from(slots))
+    theta = compiled.theta_from(slots)
     grad = np.zeros(max(1, compiled.nslots))
     value = np.zeros(1)
     weights = None
-    wp = None
     if isinstance(objective, BatchExpectationObjective):
         weights = np.ascontiguousarray(objective.sample_weights())
-        wp = N.dptr(weights)
-    rc = N.lib().mb_adjoint(compiled.handle, objective.observable.handle().handle, state.handle, N.dptr(theta),
-                            theta.size, wp, method.checkpoint_every, N.dptr(value), N.dptr(grad))
+    rc = N.lib().mb_adjoint(compiled.handle, objective.observable.handle().handle, state.handle, N.ptr(theta),
+                            theta.size, None if weights is None else N.ptr(weights), method.checkpoint_every,
+                            N.ptr(value), N.ptr(grad))
     N.check(rc, "value_and_gradient")
-    slot_grad = np.zeros(compiled.nparams)
-    for i, s in enumerate(compiled.slot_map):
-        if s >= 0:
-            slot_grad[i] = grad[s]
-    return float(value[0]), accumulate_parameter_gradients(objective.parameter_map, slot_grad)
+    return float(value[0]), accumulate_parameter_gradients(objective.parameter_map, compiled.gradient_from(grad))
 
 
 def value_and_pullback(method, objective, values):

@@ -7,6 +7,7 @@ significant local bit.
 """
 from __future__ import annotations
 
+import itertools
 import weakref
 
 import numpy as np
@@ -92,6 +93,7 @@ class QubitsOperator:
             terms = [terms]
         self.terms = [QubitsTerm(t.positions, t.op, t.coeff) for t in terms]
         self._handle = None
+        self._facts = (None, None)
 
     def add(self, term: QubitsTerm):
         self.terms.append(QubitsTerm(term.positions, term.op, term.coeff))
@@ -144,7 +146,22 @@ class QubitsOperator:
             out += t.coeff * m
         return out
 
+    def facts(self):
+        """(Hermitian, highest site, most sites of a term), kept under the terms' values."""
+        terms = self.terms
+        try:
+            key = (tuple([tuple(t.positions) for t in terms]), tuple([t.coeff for t in terms]),
+                   b"".join(itertools.chain.from_iterable([t.op for t in terms])))
+        except (BufferError, TypeError, ValueError):
+            key = None
+        if key is None or self._facts[0] != key:
+            self._facts = (key, (self._check_hermitian(), self.nqubits(), max((len(t.positions) for t in terms), default=0)))
+        return self._facts[1]
+
     def is_hermitian(self):
+        return self.facts()[0]
+
+    def _check_hermitian(self):
         keys = {}
         for t in self.terms:
             key = tuple(t.positions)
