@@ -93,7 +93,7 @@ class QubitsOperator:
             terms = [terms]
         self.terms = [QubitsTerm(t.positions, t.op, t.coeff) for t in terms]
         self._handle = None
-        self._facts = (None, None)
+        self._hermitian = (None, None)
 
     def add(self, term: QubitsTerm):
         self.terms.append(QubitsTerm(term.positions, term.op, term.coeff))
@@ -146,22 +146,32 @@ class QubitsOperator:
             out += t.coeff * m
         return out
 
-    def facts(self):
-        """(Hermitian, highest site, most sites of a term), kept under the terms' values."""
+    def _values(self):
+        """The terms by value (None when a local matrix has no flat bytes)."""
         terms = self.terms
         try:
-            key = (tuple([tuple(t.positions) for t in terms]), tuple([t.coeff for t in terms]),
-                   b"".join(itertools.chain.from_iterable([t.op for t in terms])))
+            return (tuple([tuple(t.positions) for t in terms]), tuple([t.coeff for t in terms]),
+                    b"".join(itertools.chain.from_iterable([t.op for t in terms])))
         except (BufferError, TypeError, ValueError):
-            key = None
-        if key is None or self._facts[0] != key:
-            self._facts = (key, (self._check_hermitian(), self.nqubits(), max((len(t.positions) for t in terms), default=0)))
-        return self._facts[1]
+            return None
+
+    def reach(self):
+        """(highest site, most sites of a term)."""
+        at = [t.positions for t in self.terms]
+        return max((max(p) for p in at if p), default=0), max(map(len, at), default=0)
 
     def is_hermitian(self):
-        return self.facts()[0]
+        """Kept under the terms' values."""
+        key = self._values()
+        if key is None or self._hermitian[0] != key:
+            self._hermitian = (key, self._check_hermitian())
+        return self._hermitian[1]
 
     def _check_hermitian(self):
+        if all(np.imag(t.coeff) == 0 for t in self.terms):
+            m = np.array([o for t in self.terms for o in t.op]).reshape(-1, 2, 2)
+            if np.array_equal(m, m.conj().transpose(0, 2, 1)):
+                return True      # real combinations of products of Hermitian matrices
         keys = {}
         for t in self.terms:
             key = tuple(t.positions)
