@@ -29,6 +29,9 @@ enum MopType : int16_t {
                   // population/coherence pattern of depolarizing, damping and dephasing channels:
                   // row bit r0, column bit r1, populations x00' = a x00 + b x11, x11' = e x00 +
                   // f x11, coherences x10' = c x10, x01' = d x01 (real parts of off[0..5] = a..f)
+  MOP_TAN = 12,   // real rotation c [[1,-t],[t,1]] on r0 without its factor: x -= t*y, y += t*x with
+                  // off[0] = (t, c); the factors of a pass are gathered into its MOP_SCALE
+  MOP_SCALE = 13, // every amplitude times Re off[0]
 };
 
 // Matrix offsets with this bit set index the schedule's own table of derived coefficients

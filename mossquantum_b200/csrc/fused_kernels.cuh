@@ -107,6 +107,18 @@ __device__ __forceinline__ void lift(double2 (&v)[1 << R], double mt, double s) 
     }
 }
 
+// Rotation in tangent form without its factor: x -= t*y, y += t*x.
+template <int R, int K>
+__device__ __forceinline__ void tang(double2 (&v)[1 << R], double t) {
+#pragma unroll
+  for (int j = 0; j < (1 << R); ++j)
+    if (!((j >> K) & 1)) {
+      const double2 x = v[j], y = v[j | (1 << K)];
+      v[j] = make_double2(fma(-t, y.x, x.x), fma(-t, y.y, x.y));
+      v[j | (1 << K)] = make_double2(fma(t, x.x, y.x), fma(t, x.y, y.y));
+    }
+}
+
 template <int R, int K>
 __device__ __forceinline__ void ctrl(double2 (&a)[1 << R], double2 m00, double2 m10, double2 m01, double2 m11,
                                      const MOp* __restrict__ op, int nsel, uint64_t lbase, const int* reg,
@@ -264,6 +276,19 @@ __device__ __forceinline__ void run_mops(double2 (&a)[1 << R], const MOp* __rest
         FK_CASE_K(R, 3, (lift<R, KK>(a, ts.x, ts.y)))
         FK_CASE_K(R, 4, (lift<R, KK>(a, ts.x, ts.y)))
       }
+    } else if (type == MOP_TAN) {
+      const double tn = ldm(m, xt, op->off[0], 0).x;
+      switch (r0) {
+        FK_CASE_K(R, 0, (tang<R, KK>(a, tn)))
+        FK_CASE_K(R, 1, (tang<R, KK>(a, tn)))
+        FK_CASE_K(R, 2, (tang<R, KK>(a, tn)))
+        FK_CASE_K(R, 3, (tang<R, KK>(a, tn)))
+        FK_CASE_K(R, 4, (tang<R, KK>(a, tn)))
+      }
+    } else if (type == MOP_SCALE) {
+      const double sc = ldm(m, xt, op->off[0], 0).x;
+#pragma unroll
+      for (int j = 0; j < (1 << R); ++j) a[j] = make_double2(sc * a[j].x, sc * a[j].y);
     } else if (type == MOP_RROT || type == MOP_IROT) {
       const double2 m00 = ldm(m, xt, op->off[0], conj), m10 = ldm(m, xt, op->off[1], conj);
       const double2 m01 = ldm(m, xt, op->off[2], conj), m11 = ldm(m, xt, op->off[3], conj);

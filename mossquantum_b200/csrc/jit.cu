@@ -290,6 +290,26 @@ struct StageGen {
         o << "}\n";
         break;
       }
+      case MOP_TAN: {
+        // x -= t*y; y += t*x (per component), from the old values
+        const int b = 1 << m.r0;
+        o << "{ const double tn = (" << ldm(m, 0) << ").x;\n";
+        for (int j = 0; j < A; ++j)
+          if (!(j & b)) {
+            const std::string x = v(j), y = v(j | b);
+            o << "  { const double2 ux = " << x << "; " << x << ".x = fma(-tn, " << y << ".x, ux.x); " << x << ".y = fma(-tn, "
+              << y << ".y, ux.y); " << y << ".x = fma(tn, ux.x, " << y << ".x); " << y << ".y = fma(tn, ux.y, " << y
+              << ".y); }\n";
+          }
+        o << "}\n";
+        break;
+      }
+      case MOP_SCALE: {
+        o << "{ const double sc = (" << ldm(m, 0) << ").x;\n";
+        for (int j = 0; j < A; ++j) o << "  " << v(j) << ".x *= sc; " << v(j) << ".y *= sc;\n";
+        o << "}\n";
+        break;
+      }
       case MOP_CTRL: {
         const int b = 1 << m.r0;
         int need;
@@ -608,7 +628,7 @@ static SharedMats shared_mats(const Pass& p, bool with_params) {
     cur = &m;
     switch (m.type) {
       case MOP_U1: case MOP_CTRL: case MOP_RROT: case MOP_IROT: for (int e = 0; e < 4; ++e) add(e); break;
-      case MOP_LIFT: add(0); break;
+      case MOP_LIFT: case MOP_TAN: case MOP_SCALE: add(0); break;
       case MOP_U2: for (int e = 0; e < 16; ++e) add(e); break;
       case MOP_CHAN: for (int e = 0; e < 6; ++e) add(e); break;
       case MOP_DIAG: for (int e = 0; e < (1 << m.nsel); ++e) if ((m.active >> e) & 1) add(e); break;
@@ -638,7 +658,7 @@ static SharedMats per_sample_mats(const Pass& p) {
     cur = &m;
     switch (m.type) {
       case MOP_U1: case MOP_CTRL: case MOP_RROT: case MOP_IROT: for (int e = 0; e < 4; ++e) add(e); break;
-      case MOP_LIFT: add(0); break;
+      case MOP_LIFT: case MOP_TAN: case MOP_SCALE: add(0); break;
       case MOP_U2: for (int e = 0; e < 16; ++e) add(e); break;
       case MOP_DIAG: for (int e = 0; e < (1 << m.nsel); ++e) if ((m.active >> e) & 1) add(e); break;
       case MOP_CPHASE: if (!m.r1) add(0); break;
@@ -1108,7 +1128,7 @@ static SharedMats uneven_mats(const Pass& p) {
   };
   for (const MOp& m : p.mops) switch (m.type) {
       case MOP_U1: case MOP_CTRL: case MOP_RROT: case MOP_IROT: for (int e = 0; e < 4; ++e) add(m, e); break;
-      case MOP_LIFT: add(m, 0); break;
+      case MOP_LIFT: case MOP_TAN: case MOP_SCALE: add(m, 0); break;
       case MOP_U2: for (int e = 0; e < 16; ++e) add(m, e); break;
       case MOP_CHAN: for (int e = 0; e < 6; ++e) add(m, e); break;
       case MOP_DIAG: for (int e = 0; e < (1 << m.nsel); ++e) if ((m.active >> e) & 1) add(m, e); break;
