@@ -84,6 +84,36 @@ std::string jit_pauli_source(const PauliJitPass& p, int max_vals);
 inline size_t pauli_jit_shm(int nr) { return (size_t(16) << (5 + nr)) * (nr <= 5 ? 2 : 1); }
 int jit_launch_pauli(CUfunction fn, const double2* v, const double2* coef, int64_t tps, double2* partials,
                      unsigned* counters, double2* out, int grid, int batch, size_t shm, cudaStream_t st);
+// One pass of a Pauli-string expectation as register stages over a tile of 2^t amplitudes
+// (mbk_psum): every stage holds 16 amplitudes per thread over four tile bits, and a flip group whose
+// mask lies in those bits finds both amplitudes of a pair in registers.
+struct PsumString {
+  int s;            // coefficient index
+  int zr;           // Z mask over the stage's register bits
+  uint32_t zt;      // over the other tile bits (tile-local)
+  uint64_t zh;      // over the global bits outside the tile
+  bool odd;         // odd number of Y (its coefficient multiplies i Im instead of Re)
+  bool re, im;      // the coefficient has a real / imaginary part
+};
+struct PsumGroup {
+  int xl;           // flip mask (tile-local); 0 for the diagonal
+  bool far;         // not inside the stage's register bits: partners read from the tile
+  std::vector<PsumString> strings;
+};
+struct PsumStage {
+  int reg[4];       // tile-local bits in registers, ascending
+  std::vector<PsumGroup> groups;
+};
+struct PsumPass {
+  int n, t;
+  std::vector<int> bits;   // tile-local bit -> global bit, ascending, bits 0..2 first
+  std::vector<PsumStage> stages;
+};
+inline int psum_threads(int t) { return 1 << (t - 4); }
+inline int psum_ctas(int t) { return t >= 12 ? 2 : t == 11 ? 4 : 8; }
+std::string jit_psum_source(const PsumPass& p);
+int jit_launch_psum(CUfunction fn, const double2* v, const double2* coef, int64_t tps, double2* partials,
+                    unsigned* counters, double2* out, int grid, int batch, int t, cudaStream_t st);
 int jit_launch_reg(CUfunction fn, double2* v, const double2* tab, const double2* xtab, const double2* xtabs,
                    int64_t xrow, int64_t tstride, int64_t groups, int nsamples, int grid, cudaStream_t st);
 }  // namespace mb

@@ -72,6 +72,8 @@ struct PauliProgram {
   double2* d_tables = nullptr;
   std::vector<void*> jit;        // per pass: specialised expectation kernel (mbk_pauli) or null
   double2* d_coef = nullptr;     // the observable's string coefficients, for the specialised kernels
+  int psum_t = 0;                // tile bits of the staged passes, when the program has them
+  std::vector<void*> psum;       // staged expectation kernels (mbk_psum), one per pass
 };
 
 struct PauliData {
@@ -507,6 +509,7 @@ void pauli_free(mb_observable o) {
     dev_free(p->d_coef);
     for (void* f : p->jit)
       if (f) jit_release(f);
+    for (void* f : p->psum) jit_release(f);
     delete p;
   }
   delete o->pauli;
@@ -515,8 +518,160 @@ void pauli_free(mb_observable o) {
 
 thread_local bool t_pauli_compile = true;
 
-// Specialised kernels (mbk_pauli) for the passes of a program from MB_PAULI_JIT_MIN_BITS qubits
-// (default 14; MB_PAULI_JIT=0 disables them). A pass whose per-thread factors would take too
+// Staged passes (mbk_psum) of an observable on n qubits, or empty when a flip mask does not fit a
+// tile. Tiles hold bits 0..2 (whole 128-byte lines) and any others: each pass takes flip masks in
+// ascending order while their bits fit, its stages take them in the same way into four register
+// bits (a mask wider than that reads its partners from the tile). A diagonal string goes to a stage
+// that holds all its bits in registers where one does, else to the stage that leaves out the
+// fewest. Tiles of 2^12 amplitudes from 20 qubits, down to 2^10 so that small states keep 256 of
+// them.
+static std::vector<PsumPass> psum_plan(const PauliData* pd, int n) {
+  std::vector<PsumPass> passes;
+  const int t = std::max(10, std::min(12, n - 8));
+  std::vector<int> rem;
+  int diag = -1;
+  for (size_t g = 0; g < pd->groups.size(); ++g) {
+    const uint64_t x = pd->groups[g].first;
+    if (__builtin_popcountll(x & ~uint64_t(7)) > t - 3) return {};
+    if (x == 0) diag = int(g);
+    else rem.push_back(int(g));
+  }
+  auto make_string = [&](const PsumPass& p, const PsumStage& st, int s, uint64_t x) {
+    PsumString out{};
+    const PString& ps = pd->strings[s];
+    out.s = s;
+    uint64_t z = ps.z;
+    for (int l = 0; l < t; ++l) {
+      if (!((z >> p.bits[l]) & 1)) continue;
+      z &= ~(uint64_t(1) << p.bits[l]);
+      const int* r = std::find(st.reg, st.reg + 4, l);
+      if (r != st.reg + 4) out.zr |= 1 << (r - st.reg);
+      else out.zt |= 1u << l;
+    }
+    out.zh = z;
+    out.odd = __builtin_popcountll(x & ps.z) & 1;
+    out.re = ps.c.x != 0.0;
+    out.im = ps.c.y != 0.0;
+    return out;
+  };
+  while (!rem.empty() || passes.empty()) {
+    PsumPass p;
+    p.n = n;
+    p.t = t;
+    uint64_t mask = 7;
+    for (int g : rem)
+      if (__builtin_popcountll(mask | pd->groups[g].first) <= t) mask |= pd->groups[g].first;
+    for (int q = 3; q < n && __builtin_popcountll(mask) < t; ++q) mask |= uint64_t(1) << q;
+    for (int q = 0; q < n; ++q)
+      if ((mask >> q) & 1) p.bits.push_back(q);
+    std::vector<std::pair<int, int>> take;   // (group, tile-local flip mask)
+    std::vector<int> left;
+    for (int g : rem) {
+      const uint64_t x = pd->groups[g].first;
+      if (x & ~mask) {
+        left.push_back(g);
+        continue;
+      }
+      int xl = 0;
+      for (int l = 0; l < t; ++l)
+        if ((x >> p.bits[l]) & 1) xl |= 1 << l;
+      take.push_back({g, xl});
+    }
+    do {
+      PsumStage st{};
+      int rm = 0;
+      for (auto& q : take)
+        if (__builtin_popcount(unsigned(rm | q.second)) <= 4) rm |= q.second;
+      for (int l = t - 1; l >= 0 && __builtin_popcount(unsigned(rm)) < 4; --l) rm |= 1 << l;
+      for (int l = 0, k = 0; l < t; ++l)
+        if ((rm >> l) & 1) st.reg[k++] = l;
+      std::vector<std::pair<int, int>> later;
+      bool placed = false;
+      for (size_t i = 0; i < take.size(); ++i) {
+        const bool in = (take[i].second & ~rm) == 0;
+        if (!in && !(i == 0 && __builtin_popcount(unsigned(take[i].second)) > 4)) {
+          later.push_back(take[i]);
+          continue;
+        }
+        placed = true;
+        PsumGroup g{take[i].second, !in, {}};
+        const auto& src = pd->groups[take[i].first];
+        for (int s = src.second.first; s < src.second.first + src.second.second; ++s)
+          g.strings.push_back(make_string(p, st, s, src.first));
+        st.groups.push_back(g);
+      }
+      if (!placed && !take.empty()) return {};
+      p.stages.push_back(st);
+      take.swap(later);
+    } while (!take.empty());
+    passes.push_back(p);
+    rem.swap(left);
+  }
+  if (diag >= 0) {
+    const auto& src = pd->groups[diag];
+    std::map<std::pair<int, int>, PsumGroup> at;
+    for (int s = src.second.first; s < src.second.first + src.second.second; ++s) {
+      int best = 1 << 20;
+      std::pair<int, int> where{0, 0};
+      for (size_t i = 0; i < passes.size(); ++i)
+        for (size_t k = 0; k < passes[i].stages.size(); ++k) {
+          const PsumString q = make_string(passes[i], passes[i].stages[k], s, 0);
+          // bits outside the registers cost a sign per thread, the pass's first string of a stage the
+          // sums themselves
+          const int cost = 4 * __builtin_popcount(q.zt) + 4 * __builtin_popcountll(q.zh) +
+                           (at.count({int(i), int(k)}) ? 0 : 1);
+          if (cost < best) best = cost, where = {int(i), int(k)};
+        }
+      PsumGroup& g = at[where];
+      g.xl = 0;
+      g.far = false;
+      g.strings.push_back(make_string(passes[where.first], passes[where.first].stages[where.second], s, 0));
+    }
+    for (auto& kv : at) passes[kv.first.first].stages[kv.first.second].groups.push_back(kv.second);
+  }
+  return passes;
+}
+
+static int pauli_coefficients(PauliData* pd, PauliProgram* P) {
+  if (P->d_coef) return MB_OK;
+  std::vector<double2> coef;
+  for (const PString& ps : pd->strings) coef.push_back(ps.c);
+  if (int rc = dev_alloc((void**)&P->d_coef, sizeof(double2) * coef.size())) return rc;
+  MB_CHECK_CUDA(cudaMemcpyAsync(P->d_coef, coef.data(), sizeof(double2) * coef.size(), cudaMemcpyHostToDevice, g_ctx.stream));
+  MB_CHECK_CUDA(cudaStreamSynchronize(g_ctx.stream));
+  return MB_OK;
+}
+
+// Compiles the staged passes of a program; false leaves it as it was (no placement, no compiler,
+// or a kernel that spills).
+static bool pauli_stage(PauliData* pd, PauliProgram* P) {
+  const std::vector<PsumPass> plan = psum_plan(pd, P->n);
+  if (plan.empty()) return false;
+  std::vector<std::string> src;
+  for (const PsumPass& p : plan) {
+    src.push_back(jit_psum_source(p));
+    if (src.back().empty() || src.back().size() > (size_t(256) << 10)) return false;
+  }
+  if (pauli_coefficients(pd, P) != MB_OK) return false;
+  std::vector<CUfunction> fns;
+  std::string err;
+  if (jit_prepare(src, fns, &err, 0.0) != MB_OK) {
+    if (getenv("MB_JIT_VERBOSE")) fprintf(stderr, "mossb200: staged Pauli passes: %s\n", err.c_str());
+    return false;
+  }
+  for (CUfunction f : fns)
+    if (!f || jit_local_bytes((void*)f) != 0) return false;
+  for (CUfunction f : fns) {
+    jit_retain((void*)f);
+    P->psum.push_back((void*)f);
+  }
+  P->psum_t = plan[0].t;
+  return true;
+}
+
+// Specialised kernels for a program from MB_PAULI_JIT_MIN_BITS qubits (default 14; MB_PAULI_JIT=0
+// disables them): the staged passes where every flip mask fits a tile and no kernel spills, else one
+// mbk_pauli per pass (MB_PAULI_STAGED=0 goes straight to those). A pass whose per-thread factors would take too
 // many registers, or whose kernel does not compile, keeps the interpreter kernel, and so do
 // programs built on a thread that may not compile (the serving loop: a request's observable
 // is often new, and neither NVRTC nor the source generation belongs on its path).
@@ -526,6 +681,8 @@ static void pauli_specialise(PauliData* pd, PauliProgram* P, const std::vector<P
   const int min_bits = getenv("MB_PAULI_JIT_MIN_BITS") ? atoi(getenv("MB_PAULI_JIT_MIN_BITS")) : 14;
   const char* e = getenv("MB_PAULI_JIT");
   if ((e && atoi(e) == 0) || P->n < min_bits || !t_pauli_compile || !jit_available() || pd->strings.empty()) return;
+  const char* staged = getenv("MB_PAULI_STAGED");
+  if (!(staged && atoi(staged) == 0) && pauli_stage(pd, P)) return;
   std::vector<std::string> src;
   std::vector<size_t> which;
   // Passes of 2^12-amplitude tiles (from 24 qubits) keep the interpreter unless
@@ -563,13 +720,7 @@ static void pauli_specialise(PauliData* pd, PauliProgram* P, const std::vector<P
     which.push_back(i);
   }
   if (src.empty()) return;
-  std::vector<double2> coef;
-  for (const PString& ps : pd->strings) coef.push_back(ps.c);
-  if (dev_alloc((void**)&P->d_coef, sizeof(double2) * coef.size()) != MB_OK) return;
-  if (cudaMemcpyAsync(P->d_coef, coef.data(), sizeof(double2) * coef.size(), cudaMemcpyHostToDevice, g_ctx.stream) !=
-          cudaSuccess ||
-      cudaStreamSynchronize(g_ctx.stream) != cudaSuccess)
-    return;
+  if (pauli_coefficients(pd, P) != MB_OK) return;
   std::vector<CUfunction> fns;
   std::string err;
   if (jit_prepare(src, fns, &err, 0.0) != MB_OK) {
@@ -748,6 +899,25 @@ int expect_pauli(mb_observable o, mb_state s, double2* out) {
   if (!P) return expect_keys(o, s, out);
   cudaStream_t st = g_ctx.stream;
   MB_CHECK_CUDA(cudaMemsetAsync(out, 0, sizeof(double2) * s->batch, st));
+  if (!P->psum.empty()) {
+    const int64_t tps = int64_t(1) << (s->n - P->psum_t);
+    // every CTA the SMs hold, shared out over the samples
+    const int64_t room = int64_t(g_ctx.sm_count) * psum_ctas(P->psum_t);
+    const int G = int(std::min<int64_t>(tps, std::max<int64_t>(1, std::min<int64_t>((room + s->batch - 1) / s->batch,
+                                                                                g_ctx.partials_cap / s->batch))));
+    if (int64_t(G) * s->batch > g_ctx.partials_cap || s->batch > g_ctx.ncounters) {
+      set_error("reduction workspace too small for %d samples", s->batch);
+      return MB_EUNSUPPORTED;
+    }
+    for (void* f : P->psum) {
+      ProfScope ps("mbk_pauli", 16.0 * double(s->elems) * s->batch, st);
+      if (int rc = jit_launch_psum((CUfunction)f, s->d, P->d_coef, tps, g_ctx.partials, g_ctx.counters, out, G, s->batch,
+                                   P->psum_t, st))
+        return rc;
+      MB_LAUNCHED();
+    }
+    return MB_OK;
+  }
   for (size_t i = 0; i < P->passes.size(); ++i) {
     const PPassArgs& pa = P->passes[i];
     if (pa.ngroups == 0) continue;
