@@ -12,7 +12,7 @@
 // promoted first, DensityMatrix(psi), execution/channels.jl:19); this gives the same
 // parameter gradient as promoting at the first channel.
 // Batches of density matrices enter as their weighted sum (the loss is linear in them).
-// Fused paths: pure states (one sample) and density matrices run the reverse as dual-state passes (y and Δ tiles together, gradients accumulated in the
+// Fused paths: pure states and density matrices run the reverse as dual-state passes (y and Δ tiles together, gradients accumulated in the
 // pass). On density matrices a single-qubit channel is reversed by S' on Δ and S^-1 on y (the
 // input is uncomputed instead of recomputed); segments keep the product of ||S^-1||_2 within
 // 100 and y is reset to the segment's checkpoint after each, which bounds the rounding error.
@@ -263,16 +263,17 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
     MB_CHECK_CUDA(cudaMemcpyAsync(y.p, init->d, sbytes, cudaMemcpyDeviceToDevice, st));
   }
 
-  // Fused path: pure single states with unitary circuits (specialised dual-state passes).
+  // Fused path: pure states with unitary circuits (specialised dual-state passes).
   const int nops_all = int(c->ops.size());
-  if (!is_dm && B == 1 && !c->has_channel && n >= 9 && nops_all > 0 && !plain_only) {
+  if (!is_dm && !c->has_channel && n >= 9 && nops_all > 0 && !plain_only) {
     const int kf = checkpoint_every > 0 ? checkpoint_every : nops_all;
     const int Sf = (nops_all + kf - 1) / kf;
     std::vector<Schedule*> adj(Sf, nullptr), fwd(Sf, nullptr);
     bool ok = true;
     for (int s2 = 0; s2 < Sf && ok; ++s2) {
       const int lo = s2 * kf, hi = std::min(nops_all, (s2 + 1) * kf);
-      ok = adjoint_prepare(c, n, lo, hi, &adj[s2]) == MB_OK && get_schedule_ex(c, n, 0, 0, lo, hi, 1, &fwd[s2]) == MB_OK;
+      ok = adjoint_prepare(c, n, lo, hi, &adj[s2], 0, B) == MB_OK &&
+           get_schedule_ex(c, n, 0, 0, lo, hi, B, &fwd[s2]) == MB_OK;
     }
     if (ok) {
       std::vector<std::unique_ptr<Buf>> ck(Sf);
@@ -282,26 +283,29 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
           if ((rc = ck[s2]->alloc(sbytes))) return rc;
           MB_CHECK_CUDA(cudaMemcpyAsync(ck[s2]->p, y.p, sbytes, cudaMemcpyDeviceToDevice, st));
         }
-        if ((rc = run_schedule(c, fwd[s2], y.p, 1, 0))) return rc;
+        if ((rc = run_schedule(c, fwd[s2], y.p, B, 0))) return rc;
       }
       mb_state_s view;
-      view.kind = MB_PURE;
+      view.kind = batched ? MB_BATCH_PURE : MB_PURE;
       view.n = n;
-      view.batch = 1;
+      view.batch = B;
       view.dim = int64_t(1) << n;
       view.elems = elems;
       view.d = y.p;
       if ((rc = o->pauli_ok ? expect_pauli(o, &view) : expect_keys(o, &view))) return rc;
-      double2 r0;
-      MB_CHECK_CUDA(cudaMemcpyAsync(&r0, g_ctx.results, sizeof(double2), cudaMemcpyDeviceToHost, st));
+      std::vector<double2> r(B);
+      MB_CHECK_CUDA(cudaMemcpyAsync(r.data(), g_ctx.results, sizeof(double2) * B, cudaMemcpyDeviceToHost, st));
       MB_CHECK_CUDA(cudaStreamSynchronize(st));
-      *value = w[0] * r0.x;
+      *value = 0.0;
+      for (int b = 0; b < B; ++b) *value += w[b] * r[b].x;
       bool seeded = false;
-      if (o->pauli_ok && (rc = pauli_apply(o, y.p, delta.p, n, 1, 2.0, &seeded))) return rc;
+      if (o->pauli_ok && (rc = pauli_apply(o, y.p, delta.p, n, B, 2.0, &seeded))) return rc;
       if (!seeded) {
-        if ((rc = observable_apply(o, y.p, delta.p, n, 0, 1))) return rc;
-        if ((rc = launch_scale(delta.p, elems, 2.0, st))) return rc;
+        if ((rc = observable_apply(o, y.p, delta.p, n, 0, B))) return rc;
+        if ((rc = launch_scale(delta.p, elems * B, 2.0, st))) return rc;
       }
+      // each sample's adjoint carries its weight, so the sweep's sums are the weighted gradient
+      if (B > 1 && (rc = launch_scale_samples(delta.p, elems, B, reinterpret_cast<const double*>(d_w.p), st))) return rc;
       for (int s2 = Sf - 1; s2 >= 0; --s2) {
         if ((rc = run_adjoint_schedule(c, adj[s2], y.p, delta.p, d_g))) return rc;
         if (ck[s2]) MB_CHECK_CUDA(cudaMemcpyAsync(y.p, ck[s2]->p, sbytes, cudaMemcpyDeviceToDevice, st));
@@ -309,7 +313,7 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
       std::vector<double> gh(std::max(1, c->nslots));
       if (c->nslots) MB_CHECK_CUDA(cudaMemcpyAsync(gh.data(), d_g, sizeof(double) * c->nslots, cudaMemcpyDeviceToHost, st));
       MB_CHECK_CUDA(cudaStreamSynchronize(st));
-      for (int q = 0; q < c->nslots; ++q) grad[q] = w[0] * gh[q];
+      for (int q = 0; q < c->nslots; ++q) grad[q] = B > 1 ? gh[q] : w[0] * gh[q];
       return MB_OK;
     }
   }

@@ -366,7 +366,10 @@ struct FOp {
   uint32_t active = 0;
   int conj = 0, param = 0;
   bool neg = false;           // MOP_CPHASE with factor -1 (a sign flip)
-  int slot = -1;              // MOP_GRAD / MOP_GRADP: parameter slot
+  int slot = -1;              // MOP_GRAD / MOP_GRADP / MOP_CROSS: (first) accumulator of the schedule
+  int src = -1;               // reverse sweeps: the instruction this op undoes
+  int grad = -1;              // reverse sweeps: the instruction whose gradient follows this op
+  int run = -1;               // reverse sweeps: the schedule's run that a fused op undoes
   int pauli = 0;              // MOP_GRADP: generator code (1 X, 2 Y, 3 Z, 4 PHASE)
   int only = 0;               // reverse sweeps: 0 both states, 1 y only, 2 delta only
   // plain fallback
@@ -382,7 +385,20 @@ struct FOp {
   double scale = 1.0;         // MOP_TAN: the factor c left to the pass's MOP_SCALE
 };
 
+// Reverse sweeps: what a gradient is formed from once the passes have run. kind 0: accumulator acc;
+// kind 1: the four cross sums from acc on and the gates of a run, undone in the order first ..
+// first + pos, the last of which carries the parameter with generator gen_off.
+struct AccRec {
+  int kind, acc, slot, first, pos, gen_off;
+};
+
 struct Schedule {
+  std::vector<std::vector<int>> runs;   // instructions of each fused run, in the order of undoing
+  std::vector<AccRec> accs;
+  std::vector<int> run_mats;            // table offsets of the runs' gate matrices
+  int nacc = 0;
+  AccRec* d_accs = nullptr;
+  int* d_run_mats = nullptr;
   std::vector<double2> xtab;      // derived coefficients (kXtabFlag offsets), the same for every sample
   double2* d_xtab = nullptr;      // xtab, then nsamples rows of xrow per-sample entries
   int xrow = 0;                   // per-sample entries (fused products) per row
@@ -425,6 +441,7 @@ static double mop_flops(const MOp& m) {
     case MOP_TAN: return 4.0;                  // two
     case MOP_SCALE: return 2.0;
     case MOP_GRADP: return 4.0;                // two multiply-adds per amplitude
+    case MOP_CROSS: return 12.0;               // six
     case MOP_CHAN: return 4.0;                 // 12 real multiply-adds per 4 amplitudes
     default: return 0.0;
   }
@@ -433,7 +450,7 @@ static double mop_flops(const MOp& m) {
 static double pass_flops_per_amp(const Pass& p, bool dual) {
   double f = 0;
   for (const MOp& m : p.mops)
-    f += (dual && m.type != MOP_GRAD && m.type != MOP_GRADP) ? 2.0 * mop_flops(m) : mop_flops(m);
+    f += (dual && m.type != MOP_GRAD && m.type != MOP_GRADP && m.type != MOP_CROSS) ? 2.0 * mop_flops(m) : mop_flops(m);
   return f;
 }
 
@@ -788,7 +805,22 @@ static void fuse_runs(mb_circuit c, std::vector<FOp>& seq, int n, bool dm, Sched
       channel |= seq[i].type == MOP_U2;
       param |= seq[i].param != 0;
     }
-    const bool worth = dm ? (channel || g.size() >= 3) : g.size() >= 2;
+    bool worth = dm ? (channel || g.size() >= 3) : g.size() >= 2;
+    if (S->adjoint) {
+      // FP64 instructions per amplitude of both states: a fused run is one complex 2x2 on each and
+      // six multiply-adds for the cross sums, whatever its length; gate by gate every rotation
+      // costs its cheap form on each and two multiply-adds for its gradient.
+      double apart = 0.0;
+      bool grads = false;
+      for (int i : g) {
+        const FOp& m = seq[i];
+        const bool gr = c->ops[m.src].gen_off >= 0;
+        grads |= gr;
+        apart += m.type == MOP_CTRLX ? 0.0 : m.type == MOP_CPHASE ? (gr ? 5.0 : 4.0)
+                 : (m.type == MOP_U1 ? 16.0 : 8.0) + (gr ? 2.0 : 0.0);
+      }
+      worth = g.size() >= 2 && apart > 16.0 + (grads ? 6.0 : 0.0);
+    }
     if (!worth) {
       g.clear();
       return;
@@ -849,6 +881,11 @@ static void fuse_runs(mb_circuit c, std::vector<FOp>& seq, int n, bool dm, Sched
       for (int e = 0; e < d * d; ++e) f.off[e] = xtab_push(&S->xtab, M[e]);
     }
     finalize_masks(f);
+    if (S->adjoint) {
+      f.run = int(S->runs.size());
+      S->runs.emplace_back();
+      for (int i : g) S->runs.back().push_back(seq[i].src);
+    }
     for (size_t k = 0; k + 1 < g.size(); ++k) drop[g[k]] = 1;
     repl.push_back({g.back(), f});
     g.clear();
@@ -1076,16 +1113,17 @@ static FOp grad_fop(const COp& op, int shift) {
 // channel S updates delta with S' and uncomputes y with S^-1 (inverted here; the caller bounds
 // the error growth with reverse_growth). Returns false when the range has an instruction the
 // passes cannot reverse.
-static bool build_adjoint_fops(mb_circuit c, int lo, int hi, std::vector<FOp>& out, int dm = 0, int n = 0,
-                               std::vector<double2>* xt = nullptr) {
+static bool build_adjoint_fops(mb_circuit c, int lo, int hi, std::vector<FOp>& out, int dm, int n, Schedule* S) {
   out.clear();
+  std::vector<double2>* xt = &S->xtab;
+  std::vector<FOp> seq;
   for (int oi = hi - 1; oi >= lo; --oi) {
     const COp& op = c->ops[oi];
     if (op.kind == MB_OP_CHANNEL) {
-      if (!dm || op.k != 1 || !xt) return false;
-      cd S[16], inv[16];
-      for (int e = 0; e < 16; ++e) S[e] = cd(c->fixed_table[op.mat_off + e].x, c->fixed_table[op.mat_off + e].y);
-      if (!invert4(S, inv)) return false;
+      if (!dm || op.k != 1) return false;
+      cd M[16], inv[16];
+      for (int e = 0; e < 16; ++e) M[e] = cd(c->fixed_table[op.mat_off + e].x, c->fixed_table[op.mat_off + e].y);
+      if (!invert4(M, inv)) return false;
       FOp d;
       d.type = MOP_U2;
       d.nb = 2;
@@ -1102,24 +1140,61 @@ static bool build_adjoint_fops(mb_circuit c, int lo, int hi, std::vector<FOp>& o
       y.conj = 0;
       y.only = 1;
       for (int e = 0; e < 16; ++e) y.off[e] = xtab_push(xt, make_double2(inv[e].real(), inv[e].imag()));
-      out.push_back(d);
-      out.push_back(y);
+      seq.push_back(d);
+      seq.push_back(y);
       continue;
     }
     if (op.kind != MB_OP_GATE) return false;
+    if (op.gen_off >= 0 && op.k > 2) return false;
     FOp u = gate_fop(c, op, 0, 0, true);
     mark_unfusable_masks(u);
-    out.push_back(u);
+    u.src = oi;
+    seq.push_back(u);
     if (dm) {
       FOp uc = gate_fop(c, op, n, 1, true);
       mark_unfusable_masks(uc);
-      out.push_back(uc);
+      seq.push_back(uc);
     }
-    if (op.gen_off >= 0) {
-      if (op.k > 2) return false;
-      out.push_back(grad_fop(op, 0));
-      if (dm) out.push_back(grad_fop(op, n));
+    if (op.gen_off >= 0) seq.back().grad = oi;   // density matrices: once both halves are undone
+  }
+  if (!dm && !getenv("MB_NO_FUSE")) fuse_runs(c, seq, n, false, S);
+  auto gradient = [&](const COp& op, int shift) {
+    FOp g = grad_fop(op, shift);
+    S->accs.push_back(AccRec{0, S->nacc, op.slot, 0, 0, 0});
+    g.slot = S->nacc++;
+    out.push_back(g);
+  };
+  for (const FOp& f : seq) {
+    if (f.run >= 0) {
+      const std::vector<int>& run = S->runs[f.run];
+      const int first = int(S->run_mats.size());
+      bool any = false;
+      for (size_t k = 0; k < run.size(); ++k) {
+        const COp& op = c->ops[run[k]];
+        S->run_mats.push_back(op.mat_off);
+        if (op.gen_off < 0) continue;
+        S->accs.push_back(AccRec{1, S->nacc, op.slot, first, int(k), op.gen_off});
+        any = true;
+      }
+      if (any) {
+        FOp g;
+        g.type = MOP_CROSS;
+        g.nb = 1;
+        g.bits[0] = g.tgt[0] = f.tgt[0];
+        g.ntgt = 1;
+        g.slot = S->nacc;
+        S->nacc += 4;
+        finalize_masks(g);
+        g.nd = g.all;
+        out.push_back(g);
+      }
+      out.push_back(f);
+      continue;
     }
+    out.push_back(f);
+    if (f.grad < 0) continue;
+    gradient(c->ops[f.grad], 0);
+    if (dm) gradient(c->ops[f.grad], n);
   }
   if (dm && !getenv("MB_NO_CHAN")) chan_forms(c, out, n, xt);
   return true;
@@ -1365,7 +1440,12 @@ static void plan_stages(const std::vector<FOp>& fops, const std::vector<int>& op
           return -1;
         };
         auto sel = [&](int gbit) { return int16_t(loc[gbit] >= 0 ? loc[gbit] : 64 + gbit); };
-        if (f.type == MOP_GRADP) {
+        if (f.type == MOP_CROSS) {
+          m.nsel = 1;
+          m.active = uint32_t(p.grad_slots.size());
+          for (int k = 0; k < 4; ++k) p.grad_slots.push_back(f.slot + k);
+          m.r0 = int16_t(regidx(f.tgt[0]));
+        } else if (f.type == MOP_GRADP) {
           m.nsel = 1;
           m.active = uint32_t(p.grad_slots.size());
           p.grad_slots.push_back(f.slot);
@@ -1962,7 +2042,7 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
   S->adjoint = adjoint;
   S->fuse = tu.fuse != 0;
   if (adjoint) {
-    if (!build_adjoint_fops(c, lo, hi, S->fops, dm, n, &S->xtab)) {
+    if (!build_adjoint_fops(c, lo, hi, S->fops, dm, n, S.get())) {
       set_error("the fused adjoint supports circuits with 1- and 2-qubit parameters and single-qubit channels");
       return MB_EUNSUPPORTED;
     }
@@ -1981,7 +2061,7 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
     for (const MOp& m : p.mops) {
       const bool needs = m.type == MOP_U1 || m.type == MOP_CTRL || m.type == MOP_CTRLX || m.type == MOP_U2 ||
                          m.type == MOP_GRAD || m.type == MOP_RROT || m.type == MOP_IROT || m.type == MOP_LIFT ||
-                         m.type == MOP_TAN ||
+                         m.type == MOP_TAN || m.type == MOP_CROSS ||
                          m.type == MOP_GRADP || m.type == MOP_CHAN;
       const bool two = m.type == MOP_U2 || (m.type == MOP_GRAD && m.nsel == 2);
       const bool chan_bad = m.type == MOP_CHAN && (m.r1 < 0 || m.r1 >= R || m.r1 == m.r0);
@@ -2035,6 +2115,16 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
                                   g_ctx.stream));
     MB_CHECK_CUDA(cudaMemcpyAsync(S->d_fcomps, S->fcomps.data(), sizeof(FuseComp) * S->fcomps.size(),
                                   cudaMemcpyHostToDevice, g_ctx.stream));
+  }
+  if (!S->accs.empty()) {
+    if ((rc = dev_alloc((void**)&S->d_accs, sizeof(AccRec) * S->accs.size())) ||
+        (rc = dev_alloc((void**)&S->d_run_mats, sizeof(int) * std::max<size_t>(1, S->run_mats.size()))))
+      return rc;
+    MB_CHECK_CUDA(cudaMemcpyAsync(S->d_accs, S->accs.data(), sizeof(AccRec) * S->accs.size(), cudaMemcpyHostToDevice,
+                                  g_ctx.stream));
+    if (!S->run_mats.empty())
+      MB_CHECK_CUDA(cudaMemcpyAsync(S->d_run_mats, S->run_mats.data(), sizeof(int) * S->run_mats.size(),
+                                    cudaMemcpyHostToDevice, g_ctx.stream));
   }
   MB_CHECK_CUDA(cudaStreamSynchronize(g_ctx.stream));
   if (!adjoint && !tile_only && S->R == 3 && !getenv("MB_REG_BITS")) {
@@ -2163,14 +2253,14 @@ static void prepare_jit(Schedule* S) {
   std::vector<std::string> src;
   std::vector<Pass*> who;
   // One sample: every thread reads row 0 of the matrix table, so the parametric elements can be
-  // staged in shared memory with the fixed ones.
+  // staged in shared memory with the fixed ones (reverse sweeps share the parameters in any case).
   const bool single = S->nsamples == 1;
   for (Pass& p : S->passes) {
     if (p.kind == PASS_TILE && !S->adjoint) p.ctas = tile_ctas(p.t);
     if (p.kind == PASS_TILE && S->adjoint) {
       p.ctas = adjoint_ctas(p.t, S->dm);
-      src.push_back(memo_source(pass_key(p, 1, S->R, S->N, single, p.ctas),
-                                [&] { return jit_adjoint_source(p, S->R, S->N, single, p.ctas); }));
+      src.push_back(memo_source(pass_key(p, 1, S->R, S->N, true, p.ctas),
+                                [&] { return jit_adjoint_source(p, S->R, S->N, true, p.ctas); }));
     } else if (p.kind == PASS_TILE) {
       src.push_back(memo_source(pass_key(p, 0, S->R, S->N, single, p.ctas),
                                 [&] { return jit_tile_source(p, S->R, S->N, single, p.ctas); }));
@@ -2326,6 +2416,41 @@ int run_schedule(mb_circuit c, Schedule* S, double2* v, int nsamples, int64_t ms
   return MB_OK;
 }
 
+// Gradients from a reverse sweep's accumulators. For a gate of a run, with C the cross sums of
+// delta y' after the run and V = U_k' .. U_K' (the run's gates from the last back to this one),
+// Re<y_k|D|delta_k> = Re tr(V'DV C); V'DV is anti-Hermitian like D, so four real sums of C serve.
+__global__ void k_adjoint_grads(const AccRec* __restrict__ recs, int nrecs, const int* __restrict__ mats,
+                                const double2* __restrict__ table, const double* __restrict__ acc, double* grad) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nrecs) return;
+  const AccRec r = recs[i];
+  const double* C = acc + r.acc;
+  if (r.kind == 0) {
+    atomicAdd(grad + r.slot, C[0]);
+    return;
+  }
+  // column-major 2x2 products X Y
+  auto mul = [](const double2* X, const double2* Y, double2* Z) {
+    for (int col = 0; col < 2; ++col)
+      for (int row = 0; row < 2; ++row) Z[row + 2 * col] = cfma(X[row + 2], Y[1 + 2 * col], cmul(X[row], Y[2 * col]));
+  };
+  auto adj = [](const double2* X, double2* Z) {
+    for (int col = 0; col < 2; ++col)
+      for (int row = 0; row < 2; ++row) Z[row + 2 * col] = cconj(X[col + 2 * row]);
+  };
+  double2 V[4] = {make_double2(1.0, 0.0), cz(), cz(), make_double2(1.0, 0.0)}, X[4], Z[4];
+  for (int k = 0; k <= r.pos; ++k) {
+    adj(table + mats[r.first + k], X);
+    mul(X, V, Z);
+    for (int e = 0; e < 4; ++e) V[e] = Z[e];
+  }
+  mul(table + r.gen_off, V, X);
+  adj(V, Z);
+  double2 M[4];
+  mul(Z, X, M);
+  atomicAdd(grad + r.slot, -(M[0].y * C[0] + M[3].y * C[1] + M[2].x * C[3] + M[2].y * C[2]));
+}
+
 // Reverse sweep over an adjoint schedule: U' on y and delta in every pass, gradient
 // contributions added into d_grad (one entry per parameter slot), summed over the schedule's
 // samples (stored back to back; they share the parameters).
@@ -2344,6 +2469,7 @@ int run_adjoint_schedule(mb_circuit c, Schedule* S, double2* y, double2* d, doub
     return MB_EUNSUPPORTED;
   }
   double* gpart = nullptr;
+  double* acc = nullptr;
   unsigned* gcount = nullptr;
   const int grid_max = g_ctx.sm_count * 4;
   int rc;
@@ -2352,8 +2478,20 @@ int run_adjoint_schedule(mb_circuit c, Schedule* S, double2* y, double2* d, doub
     dev_free(gpart);
     return rc;
   }
+  if ((rc = dev_alloc((void**)&acc, sizeof(double) * std::max(1, S->nacc)))) {
+    dev_free(gpart);
+    dev_free(gcount);
+    return rc;
+  }
   cudaMemsetAsync(gcount, 0, sizeof(unsigned), st);
   const int B = S->nsamples;
+  double2* xs = S->d_xtab ? S->d_xtab + S->xtab.size() : nullptr;
+  if (!S->frecs.empty()) {
+    ProfScope ps("k_fuse", 0.0, st);
+    k_fuse<<<unsigned((S->frecs.size() + 127) / 128), 128, 0, st>>>(S->d_frecs, int(S->frecs.size()), S->d_fcomps,
+                                                                     c->d_table, 0, xs, S->xrow, 1);
+    MB_LAUNCHED();
+  }
   for (const Pass& p : S->passes) {
     if (p.kind == PASS_PLAIN) {
       const FOp& f = S->fops[p.plain_fop];
@@ -2371,10 +2509,20 @@ int run_adjoint_schedule(mb_circuit c, Schedule* S, double2* y, double2* d, doub
     const int grid = int(std::min<int64_t>(ntiles, int64_t(g_ctx.sm_count) * std::min(per_sm, std::max(1, p.ctas))));
     ProfScope ps("k_adjoint_pass_jit", 64.0 * double(elems) * B, st, pass_flops_per_amp(p, true) * double(elems) * B);
     rc = jit_launch_adjoint((CUfunction)p.jit_fn, &my, &md, c->d_table, 0, tps, ntiles, g_ctx.flags + 2, gpart, gcount,
-                            d_grad, S->d_gslots + p.grad_off, S->d_xtab, threads, shm, grid, st);
+                            acc, S->d_gslots + p.grad_off, S->d_xtab, xs, threads, shm, grid, st);
     ++launch_counter();
     if (rc) break;
   }
+  if (!rc && !S->accs.empty()) {
+    k_adjoint_grads<<<unsigned((S->accs.size() + 127) / 128), 128, 0, st>>>(S->d_accs, int(S->accs.size()), S->d_run_mats,
+                                                                             c->d_table, acc, d_grad);
+    ++launch_counter();
+    if (cudaGetLastError() != cudaSuccess) {
+      set_error("gradient launch failed");
+      rc = MB_EDEVICE;
+    }
+  }
+  dev_free(acc);
   dev_free(gpart);
   dev_free(gcount);
   return rc;
@@ -2417,6 +2565,8 @@ void release_schedules(mb_circuit c) {
     dev_free(s->d_xtab);
     dev_free(s->d_frecs);
     dev_free(s->d_fcomps);
+    dev_free(s->d_accs);
+    dev_free(s->d_run_mats);
     delete s;
   }
   c->scheds.clear();
@@ -2878,7 +3028,7 @@ extern "C" int mb_schedule_info(const mb_op* ops, size_t nops, int n, int dm, in
       A.R = 3;
       if (const char* e = getenv("MB_ADJOINT_REG_BITS")) A.R = std::max(3, std::min(4, atoi(e)));
       A.adjoint = 1;
-      if (mb::build_adjoint_fops(&c, 0, int(c.ops.size()), A.fops, A.dm, n, &A.xtab)) {
+      if (mb::build_adjoint_fops(&c, 0, int(c.ops.size()), A.fops, A.dm, n, &A)) {
         mb::build_schedule(A, nsamples, false);
         int j = 0;
         for (mb::Pass& ps : A.passes) {

@@ -32,6 +32,9 @@ enum MopType : int16_t {
   MOP_TAN = 12,   // real rotation c [[1,-t],[t,1]] on r0 without its factor: x -= t*y, y += t*x with
                   // off[0] = (t, c); the factors of a pass are gathered into its MOP_SCALE
   MOP_SCALE = 13, // every amplitude times Re off[0]
+  MOP_CROSS = 14, // adjoint sweep: the four real cross sums of delta y' on register bit r0 that the
+                  // gradients of a run of gates follow from: Im C00, Im C11, Im(C01 + C10),
+                  // Re(C01 - C10); active = the first of four accumulator indices
 };
 
 // Matrix offsets with this bit set index the schedule's own table of derived coefficients
@@ -82,7 +85,7 @@ struct Pass {
   bool has_u2 = false;          // holds a 4x4 micro-op (selects the kernel variant)
   void* jit_fn = nullptr;       // specialised kernel (CUfunction) when the JIT is in use
   int ctas = 0;                 // specialised tile kernels: CTAs per SM they were compiled for
-  std::vector<int> grad_slots;  // adjoint passes: parameter slot of each gradient accumulator
+  std::vector<int> grad_slots;  // adjoint passes: the schedule's accumulator of each one in the pass
   int grad_off = 0;             // offset of grad_slots in the schedule's device slot array
   TmaGeom geom{};
   int stage_off = 0, mop_off = 0;  // offsets into the schedule's device buffers

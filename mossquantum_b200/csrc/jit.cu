@@ -890,6 +890,33 @@ static void emit_grad(std::ostringstream& o, const MOp& m, const StageGen& gy, c
   o << "  " << name << " = gs;\n}\n";
 }
 
+// The thread's part of a run's four cross sums (MOP_CROSS): 12 multiply-adds per pair.
+static void emit_cross(std::ostringstream& o, const MOp& m, const StageGen& gy, const StageGen& gd, int R,
+                       const std::vector<std::string>& s) {
+  const int b = 1 << m.r0;
+  for (int j = 0; j < (1 << R); ++j) {
+    if (j & b) continue;
+    const std::string y0 = gy.v(j), y1 = gy.v(j | b), d0 = gd.v(j), d1 = gd.v(j | b);
+    auto add = [&](const std::string& t, const char* sign, const std::string& u, const std::string& v) {
+      o << " " << t << " = fma(" << sign << u << ", " << v << ", " << t << ");";
+    };
+    o << "     ";
+    add(s[0], "", d0 + ".y", y0 + ".x");
+    add(s[1], "", d1 + ".y", y1 + ".x");
+    add(s[2], "", d0 + ".y", y1 + ".x");
+    add(s[3], "", d0 + ".x", y1 + ".x");
+    add(s[0], "-", d0 + ".x", y0 + ".y");
+    add(s[1], "-", d1 + ".x", y1 + ".y");
+    add(s[2], "-", d0 + ".x", y1 + ".y");
+    add(s[3], "", d0 + ".y", y1 + ".y");
+    add(s[2], "", d1 + ".y", y0 + ".x");
+    add(s[3], "-", d1 + ".x", y0 + ".x");
+    add(s[2], "-", d1 + ".x", y0 + ".y");
+    add(s[3], "-", d1 + ".y", y0 + ".y");
+    o << "\n";
+  }
+}
+
 // Sums k partial sums (consecutive accumulators acc0, acc0+1, ...) over the warp in one
 // butterfly: at step s the lanes with lane bit s set keep the upper half of their values and
 // send the lower half, so k values take (k - 1) + (5 - log2 k) shuffles instead of 5k. Lane L
@@ -931,8 +958,7 @@ std::string jit_adjoint_source(const Pass& p, int R, int N, bool stage_params, i
     << ") mbk_adj(const __grid_constant__ TMap tmy, "
     << "const __grid_constant__ TMap tmd, const double2* __restrict__ tab, long long tstride, long long tps, "
     << "long long ntiles, u32* err, double* gpart, u32* gcount, double* gout, const int* __restrict__ gslot, "
-    << "const double2* __restrict__ xtab) {\n";
-  o << "  const double2* __restrict__ xtabs = nullptr; (void)xtabs;\n";
+    << "const double2* __restrict__ xtab, const double2* __restrict__ xtabs) {\n";
   o << "  extern __shared__ unsigned char smem_raw[];\n  __shared__ __align__(8) u64 bar[2];\n  __shared__ int s_abort;\n"
     << "  __shared__ bool lastcta;\n";
   o << shared_mats_fill(smats);
@@ -1015,16 +1041,20 @@ std::string jit_adjoint_source(const Pass& p, int R, int N, bool stage_params, i
     int gacc0 = -1, gcount = 0;
     for (int q = 0; q < sd.nops; ++q) {
       const MOp& m = p.mops[sd.op0 + q];
-      if (m.type == MOP_GRAD || m.type == MOP_GRADP) {
-        if (int(gnames.size()) == gchunk || (gacc0 >= 0 && int(m.active) != gacc0 + int(gnames.size()))) {
-          emit_grad_reduce(o, gnames, gacc0, nw);
+      if (m.type == MOP_GRAD || m.type == MOP_GRADP || m.type == MOP_CROSS) {
+        const int need = m.type == MOP_CROSS ? 4 : 1;
+        if (int(gnames.size()) + need > std::max(gchunk, need) ||
+            (gacc0 >= 0 && int(m.active) != gacc0 + int(gnames.size()))) {
+          if (!gnames.empty()) emit_grad_reduce(o, gnames, gacc0, nw);
           gnames.clear();
         }
         if (gnames.empty()) gacc0 = int(m.active);
-        const std::string name = "gp" + std::to_string(gcount++);
-        o << "      double " << name << ";\n";
-        emit_grad(o, m, gy, gd, R, name);
-        gnames.push_back(name);
+        std::vector<std::string> names;
+        for (int k = 0; k < need; ++k) names.push_back("gp" + std::to_string(gcount++));
+        for (const std::string& name : names) o << "      double " << name << (need == 4 ? " = 0.0" : "") << ";\n";
+        if (need == 4) emit_cross(o, m, gy, gd, R, names);
+        else emit_grad(o, m, gy, gd, R, names[0]);
+        gnames.insert(gnames.end(), names.begin(), names.end());
       } else {
         if (m.only != 2) gy.emit(m);   // channels: S^-1 on y only, S' on delta only
         if (m.only != 1) gd.emit(m);
@@ -1046,8 +1076,10 @@ std::string jit_adjoint_source(const Pass& p, int R, int N, bool stage_params, i
       << "; ++w) s += gw[gi * " << nw << " + w]; gpart[(long long)gi * gridDim.x + blockIdx.x] = s; }\n";
     o << "  __threadfence();\n  __syncthreads();\n";
     o << "  if (tx == 0) lastcta = atomicAdd(gcount, 1u) == gridDim.x - 1;\n  __syncthreads();\n";
-    o << "  if (lastcta) {\n    __threadfence();\n    for (int gi = tx; gi < " << ngrad
-      << "; gi += blockDim.x) { double s = 0.0; for (unsigned c = 0; c < gridDim.x; ++c) s += __ldcg(&gpart[(long long)gi * gridDim.x + c]); atomicAdd(&gout[gslot[gi]], s); }\n";
+    // a warp per accumulator: its lanes stride over the CTAs (hundreds), then a fixed butterfly
+    o << "  if (lastcta) {\n    __threadfence();\n    for (int gi = tx >> 5; gi < " << ngrad << "; gi += " << nw
+      << ") { double s = 0.0; for (unsigned c = tx & 31u; c < gridDim.x; c += 32u) s += __ldcg(&gpart[(long long)gi * gridDim.x + c]);\n"
+      << "      for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);\n      if ((tx & 31u) == 0) gout[gslot[gi]] = s; }\n";
     o << "    __syncthreads();\n    if (tx == 0) *gcount = 0u;\n  }\n";
   }
   o << "}\n";
@@ -1057,12 +1089,13 @@ std::string jit_adjoint_source(const Pass& p, int R, int N, bool stage_params, i
 
 int jit_launch_adjoint(CUfunction fn, const CUtensorMap* my, const CUtensorMap* md, const double2* tab, int64_t tstride,
                        int64_t tps, int64_t ntiles, unsigned* err, double* gpart, unsigned* gcount, double* gout,
-                       const int* gslot, const double2* xtab, int threads, size_t shm, int grid, cudaStream_t st) {
+                       const int* gslot, const double2* xtab, const double2* xtabs, int threads, size_t shm, int grid,
+                       cudaStream_t st) {
   Drv& d = drv();
   if (d.setattr(fn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, int(shm)) != CUDA_SUCCESS) return MB_EDEVICE;
   long long ts = tstride, tp = tps, nt = ntiles;
   void* params[] = {(void*)my, (void*)md, (void*)&tab, &ts, &tp, &nt, &err, &gpart, &gcount, &gout, (void*)&gslot,
-                    (void*)&xtab};
+                    (void*)&xtab, (void*)&xtabs};
   if (d.launch(fn, grid, 1, 1, threads, 1, 1, unsigned(shm), (CUstream)st, params, nullptr) != CUDA_SUCCESS) {
     set_error("JIT adjoint launch failed");
     return MB_EDEVICE;

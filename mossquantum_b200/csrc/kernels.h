@@ -43,6 +43,8 @@ int launch_dmma(double2* v, int64_t elems, int nsamples, const Pos& pos, const d
 // ---- state utilities ---------------------------------------------------------------------
 int launch_set_basis(double2* v, int64_t elems, int nsamples, int64_t index, cudaStream_t st);
 int launch_to_density(const double2* psi, double2* rho, int n, int nsamples, cudaStream_t st);
+// v[b] *= scales[b] (device array) for every sample of elems amplitudes.
+int launch_scale_samples(double2* v, int64_t elems, int nsamples, const double* scales, cudaStream_t st);
 // out = sum_b w_b rho_b (or, for pure samples, sum_b w_b |psi_b><psi_b|); w on the device.
 int launch_weighted_density(const double2* in, bool pure, const double* w, int B, int n, double2* out, cudaStream_t st);
 int launch_identity_density(double2* rho, int n, int nsamples, cudaStream_t st);

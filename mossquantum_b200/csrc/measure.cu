@@ -38,6 +38,16 @@ __global__ void k_scale_samples(double2* __restrict__ v, int64_t elems, int nsam
   }
 }
 
+}  // namespace
+
+int launch_scale_samples(double2* v, int64_t elems, int nsamples, const double* scales, cudaStream_t st) {
+  k_scale_samples<<<grid_for(elems * nsamples, 256), 256, 0, st>>>(v, elems, nsamples, scales);
+  MB_LAUNCHED();
+  return MB_OK;
+}
+
+namespace {
+
 int check_qubit(mb_state s, int qubit) {
   if (!s) return MB_EINVAL;
   if (qubit < 0 || qubit >= s->n) {

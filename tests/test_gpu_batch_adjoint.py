@@ -62,3 +62,31 @@ def test_density_strings_match_keys(mq, monkeypatch, n, B):
         assert np.max(np.abs(got - keys)) <= 1e-11 * scale
         for b in range(B):
             assert abs(got[b] - np.trace(H.matrix(n) @ rho[:, :, b])) <= 1e-11 * scale
+
+
+@pytest.mark.parametrize("n,B,ck", [(13, 3, 0), (13, 2, 31), (14, 1, 0)])
+def test_pure_reverse_with_runs(mq, O, n, B, ck):
+    """Runs of gates undone as one 2x2 with cross sums, beside controlled and two-qubit gates that stay
+    apart, fixed gates inside runs, adjoint gates, and one parameter per gate."""
+    rng = np.random.default_rng(n + B)
+    a = lambda: float(rng.uniform(0, 2 * np.pi))
+    c = mq.QCircuit()
+    for layer in range(2):
+        for q in range(1, n + 1):
+            c.push(mq.RxGate(q, a(), isparas=True))
+            c.push([mq.HGate(q), mq.RyGate(q, a(), isparas=True).adjoint(), mq.TGate(q), mq.PHASEGate(q, a(), isparas=True)][q % 4])
+            c.push(mq.RzGate(q, a(), isparas=q % 3 != 0))
+            if q % 5 == 0:
+                c.push(mq.RxGate(q, a(), isparas=True))
+        for q in range(1, n):
+            c.push(mq.CNOTGate(q, q + 1) if q % 3 else mq.CRyGate(q + 1, q, a(), isparas=True))
+        c.push(mq.iSWAPGate(2, 9))
+    H, v = mq.QubitsOperator([mq.QubitsTerm([1, n], ["X", "Y"], 0.5), mq.QubitsTerm([4], ["Z"], -1.0)]), unit(n, B, n)
+    w = np.linspace(0.5, -0.75, B) if B > 1 else [1.0]
+    if B > 1:
+        obj = mq.BatchExpectationObjective(c, H, mq.BatchStateVector(v), reduction="weighted_sum", weights=w)
+    else:
+        obj = mq.ExpectationObjective(c, H, mq.StateVector(v[:, 0]))
+    val, g = mq.value_and_gradient(mq.AdjointGradient(checkpoint_every=ck), obj, c.active_parameters())
+    vr, gr = weighted(O, c, v, n, H, w, False)
+    assert abs(val - vr) <= 1e-11 and np.max(np.abs(g - gr)) <= 1e-10
