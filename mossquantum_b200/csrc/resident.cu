@@ -10,17 +10,23 @@
 //    t's value from a storage index, and the flip mask col[t] that toggles bit t alone. A gate on t
 //    pairs storage indexes p and p ^ col[t]; controls and Pauli strings are parities.
 //  - Runs. Consecutive gates on one qubit form a group, multiplied into one 2x2 when the angles are
-//    bound: the hardware-efficient ansatz takes n steps per layer.
+//    bound.
+//  - Stages. Groups whose targets share a frame run together, R qubits at a time: a thread holds the
+//    2^R amplitudes (of both states) that the targets span, so R groups cost one barrier and one
+//    round trip. The hardware-efficient ansatz takes n / R stages per layer.
 //  - Gradients. All gradients of a group follow from four cross sums of its pairs (k_resident's
 //    reverse); a step only stores each thread's part, and the parts are added a chunk at a time.
 // Sums have a fixed order: the same bits on every run.
-// Measured (8 qubits, 2 layers of the ansatz): value 20 us and gradient 28 us, where the plain
-// reverse took 266 launches (1.98 ms per call); 48 samples of 12 qubits, 4 layers: 220 us against
-// 732 launches (5.3 ms). Above 12 qubits the passes over HBM are the only form: two states no longer
-// fit one SM.
+// Measured (8 qubits, 2 layers of the ansatz): value 10 us and gradient 17 us of SM time (47 and 60 us
+// per call; the plain reverse took 266 launches and 2.0 ms); 48 samples of 12 qubits, 4 layers:
+// 150 us (732 launches and 5.3 ms per call before). One qubit per stage took 226 us for the last: the
+// stages are bound by barriers and shared-memory round trips, and three qubits' tuples of both
+// states are what a thread's registers hold. Above 12 qubits the passes over HBM are the only form:
+// two states no longer fit one SM.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "internal.h"
@@ -48,18 +54,26 @@ struct __align__(8) ROp {
   int32_t e[4];         // RO_U1: table offsets of m00, m10, m01, m11
 };
 
-enum RKind : uint16_t { RG_PAIR, RG_U2, RG_DIAG };
+enum RKind : uint16_t { RG_PAIRS, RG_U2, RG_DIAG };
 
+// One run of gates of a stage, on its local bit `bit`.
 struct __align__(8) RGroup {
-  uint16_t kind, nctl;
-  uint16_t ctl[4];      // parity masks of the controls (RG_DIAG: of local bits 1..4)
+  uint16_t bit, nctl;
+  uint16_t ctl[4];      // parity masks of the controls
   uint16_t cbits;       // their constants
-  uint16_t v, r;        // flip mask and parity mask of the target
-  uint16_t rc, pivot;   // parity constant; storage bit left out when pairs are counted
-  uint16_t v2, r2;      // RG_U2: second bit
-  uint16_t rc2, pivot2;
-  uint16_t op0, nops;   // RG_PAIR: gates; others: first entry in mat
+  uint16_t cm;          // four bits per control: which local flips toggle it
+  uint16_t op0, nops;
   int16_t grad;         // row of the group's cross sums, or -1
+  uint16_t pad;
+};
+
+// RG_PAIRS: groups [g0, g0 + ng) on R targets with flip masks v and parity masks r (constants rc).
+// RG_U2 / RG_DIAG: one gate without gradients, its matrix at mat[g0..] (RG_U2 on targets 0 and 1;
+// RG_DIAG with local bit 0 at r[0] and bits 1..4 at ctl).
+struct __align__(8) RStage {
+  uint16_t kind, g0, ng, rc;
+  uint16_t v[3], r[3], pivot[3];  // pivots (ascending): storage bits left out when tuples are counted
+  uint16_t ctl[4], nctl, cbits;
 };
 
 struct RAngle {
@@ -73,23 +87,30 @@ struct ResidentPlan {
   int n = 0;
   bool ok = false;
   bool unique = true;               // every slot has one gate
-  int ngroups = 0, nops = 0, ncs = 0, nmat = 0, ngrad = 0;   // ngrad: groups with gradients
+  int nstages = 0, ngroups = 0, nops = 0, ncs = 0, nmat = 0, ngrad = 0;   // ngrad: groups with gradients
   uint16_t row[kResMaxBits] = {0}, col[kResMaxBits] = {0}, rconst = 0;  // frame after the circuit
-  void* d = nullptr;                // groups, ops, angles, matrix offsets
-  size_t off_ops = 0, off_ang = 0, off_mat = 0;
+  void* d = nullptr;                // stages, groups, ops, angles, matrix offsets
+  size_t off_groups = 0, off_ops = 0, off_ang = 0, off_mat = 0;
 };
 
 namespace {
 
+// Parameters travel with the launch up to this many; more go up in a copy first.
+constexpr int kResTheta = 384;
+struct RTheta {
+  double v[kResTheta];
+};
+
 struct RArgs {
-  int n, grad, ngroups, nops, ncs, nmat, ngrad, nslots, unique, nflips, nstr, B, chunk;
+  int n, grad, nstages, ngroups, nops, ncs, nmat, ngrad, nslots, unique, nflips, nstr, B, chunk;
   uint16_t row[kResMaxBits], col[kResMaxBits], rconst;
+  const RStage* stages;
   const RGroup* groups;
   const ROp* ops;
   const RAngle* angles;
   const int* mat_off;
   const double2* table;
-  const double* theta;
+  const double* theta;              // null: in the launch's RTheta
   const double* weights;
   const double2* init;
   const PFlip* flips;
@@ -102,12 +123,6 @@ struct RArgs {
 
 __device__ __forceinline__ int rswz(int i) { return i ^ ((i >> 3) & 7); }
 __device__ __forceinline__ unsigned par(unsigned x) { return __popc(x) & 1u; }
-
-__device__ __forceinline__ bool controls_on(const RGroup& g, unsigned p) {
-  bool on = true;
-  for (int c = 0; c < g.nctl; ++c) on = on && (par(g.ctl[c] & p) ^ ((g.cbits >> c) & 1u));
-  return on;
-}
 
 struct M2 {
   double2 m00, m10, m01, m11;
@@ -153,9 +168,6 @@ __device__ __forceinline__ DD dd_fma(double a, DD b, DD c) {
 struct CDD {
   DD x, y;
 };
-struct M2DD {
-  CDD m00, m10, m01, m11;
-};
 __device__ __forceinline__ CDD wide(double2 a) { return CDD{DD{a.x, 0.0}, DD{a.y, 0.0}}; }
 __device__ __forceinline__ double2 narrow(const CDD& a) { return make_double2(a.x.h, a.y.h); }
 // a * b + c * d
@@ -164,36 +176,31 @@ __device__ __forceinline__ CDD cdot(double2 a, const CDD& b, double2 c, const CD
   return CDD{dd_fma(-c.y, d.y, dd_fma(c.x, d.x, dd_fma(-a.y, b.y, dd_fma(a.x, b.x, z)))),
              dd_fma(c.y, d.x, dd_fma(c.x, d.y, dd_fma(a.y, b.x, dd_fma(a.x, b.y, z))))};
 }
-__device__ __forceinline__ M2DD mul(const M2& a, const M2DD& b) {
-  return M2DD{cdot(a.m00, b.m00, a.m01, b.m10), cdot(a.m10, b.m00, a.m11, b.m10),
-              cdot(a.m00, b.m01, a.m01, b.m11), cdot(a.m10, b.m01, a.m11, b.m11)};
-}
 
 // Storage index of pair q: a zero inserted at the pivot.
 __device__ __forceinline__ int insert0(int q, int pivot) {
   return ((q >> pivot) << (pivot + 1)) | (q & ((1 << pivot) - 1));
 }
 
-// Element-wise diagonal and 4x4 groups (no gradients): one state.
-__device__ __noinline__ void other_group(const RGroup& g, const double2* mat, double2* s, int n, bool adj) {
+// Element-wise diagonal and 4x4 gates (no gradients): one state.
+__device__ __noinline__ void other_stage(const RStage& g, const double2* mat, double2* s, int n, bool adj) {
   if (g.kind == RG_DIAG) {
     for (int p = threadIdx.x; p < (1 << n); p += blockDim.x) {
-      unsigned idx = par(g.r & p) ^ g.rc;
+      unsigned idx = par(g.r[0] & p) ^ (g.rc & 1u);
       for (int c = 0; c < g.nctl; ++c) idx |= (par(g.ctl[c] & p) ^ ((g.cbits >> c) & 1u)) << (c + 1);
-      const double2 f = mat[g.op0 + idx];
+      const double2 f = mat[g.g0 + idx];
       s[rswz(p)] = cmul(adj ? cconj(f) : f, s[rswz(p)]);
     }
     return;
   }
-  const int lo = min(g.pivot, g.pivot2), hi = max(g.pivot, g.pivot2);
   for (int q = threadIdx.x; q < (1 << (n - 2)); q += blockDim.x) {
-    const int p = insert0(insert0(q, lo), hi);
-    const unsigned a0 = par(g.r & p) ^ g.rc, a1 = par(g.r2 & p) ^ g.rc2;
+    const int p = insert0(insert0(q, g.pivot[0]), g.pivot[1]);
+    const unsigned a0 = par(g.r[0] & p) ^ (g.rc & 1u), a1 = par(g.r[1] & p) ^ ((g.rc >> 1) & 1u);
     int at[4];
     double2 x[4];
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-      at[m] = rswz(p ^ (((m & 1) ^ a0) ? g.v : 0) ^ (((m >> 1) ^ a1) ? g.v2 : 0));
+      at[m] = rswz(p ^ (((m & 1) ^ a0) ? g.v[0] : 0) ^ (((m >> 1) ^ a1) ? g.v[1] : 0));
       x[m] = s[at[m]];
     }
 #pragma unroll
@@ -201,7 +208,7 @@ __device__ __noinline__ void other_group(const RGroup& g, const double2* mat, do
       double2 acc = cz();
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
-        const double2 u = adj ? cconj(mat[g.op0 + m + 4 * r]) : mat[g.op0 + r + 4 * m];
+        const double2 u = adj ? cconj(mat[g.g0 + m + 4 * r]) : mat[g.g0 + r + 4 * m];
         acc = cfma(u, x[m], acc);
       }
       s[at[r]] = acc;
@@ -209,12 +216,58 @@ __device__ __noinline__ void other_group(const RGroup& g, const double2* mat, do
   }
 }
 
-// PAIRS pairs per thread; the block has 2^(n-1) / PAIRS threads (at least a warp: below 6 qubits the
-// threads past the last pair carry zeros and store nothing).
-template <int PAIRS>
-__global__ void __launch_bounds__(kResMaxThreads) k_resident(const RArgs a) {
+// Which of a thread's pairs a group acts on: one bit per local index with the target bit clear.
+template <int R>
+__device__ __forceinline__ unsigned pairs_on(const RGroup& g, unsigned base) {
+  unsigned on = (1u << (1 << R)) - 1u;
+  for (int c = 0; c < g.nctl; ++c) {
+    const unsigned p0 = par(g.ctl[c] & base) ^ ((g.cbits >> c) & 1u), cm = (g.cm >> (4 * c)) & 15u;
+    unsigned ok = 0;
+#pragma unroll
+    for (int m = 0; m < (1 << R); ++m) ok |= (p0 ^ par(cm & unsigned(m))) << m;
+    on &= ok;
+  }
+  return on;
+}
+
+// ALL: every pair, without a branch between the pairs' independent chains.
+template <int R, int K, bool ALL>
+__device__ __forceinline__ void apply_bit(double2 (&a)[1 << R], const M2& m, unsigned on) {
+#pragma unroll
+  for (int j = 0; j < (1 << R); ++j)
+    if (!((j >> K) & 1) && (ALL || ((on >> j) & 1u))) apply(m, a[j], a[j | (1 << K)]);
+}
+
+// f(integral constant) for the run-time bit 0 .. R-1.
+template <int R, typename F>
+__device__ __forceinline__ void on_bit(int bit, F f) {
+  if (bit == 0) f(std::integral_constant<int, 0>());
+  if constexpr (R > 1) if (bit == 1) f(std::integral_constant<int, 1>());
+  if constexpr (R > 2) if (bit == 2) f(std::integral_constant<int, 2>());
+}
+
+template <int R, int K, bool ALL>
+__device__ __forceinline__ void cross_bit(const double2 (&y)[1 << R], const double2 (&d)[1 << R], unsigned on,
+                                          double (&s)[4]) {
+#pragma unroll
+  for (int j = 0; j < (1 << R); ++j)
+    if (!((j >> K) & 1) && (ALL || ((on >> j) & 1u))) {
+      const double2 y0 = y[j], y1 = y[j | (1 << K)], d0 = d[j], d1 = d[j | (1 << K)];
+      s[0] = fma(d0.y, y0.x, fma(-d0.x, y0.y, s[0]));
+      s[1] = fma(d1.y, y1.x, fma(-d1.x, y1.y, s[1]));
+      s[2] = fma(d0.y, y1.x, fma(-d0.x, y1.y, fma(d1.y, y0.x, fma(-d1.x, y0.y, s[2]))));
+      s[3] = fma(d0.x, y1.x, fma(d0.y, y1.y, fma(-d1.x, y0.x, fma(-d1.y, y0.y, s[3]))));
+    }
+}
+
+// A thread holds one tuple of 2^R amplitudes per state; the block has 2^(n-R) threads (at least a
+// warp: threads past the last tuple load nothing and store nothing).
+template <int R>
+__global__ void __launch_bounds__(kResMaxThreads) k_resident(const __grid_constant__ RArgs a,
+                                                             const __grid_constant__ RTheta th) {
   extern __shared__ __align__(16) unsigned char raw[];
-  const int n = a.n, dim = 1 << n, npairs = dim >> 1, T = blockDim.x, tx = threadIdx.x, b = blockIdx.x;
+  const int n = a.n, dim = 1 << n, T = blockDim.x, tx = threadIdx.x, b = blockIdx.x;
+  constexpr int A = 1 << R;
   double2* psi = reinterpret_cast<double2*>(raw);
   double2* del = psi + dim;
   M2* gm = reinterpret_cast<M2*>(del + (a.grad ? dim : 0));   // fused matrix of every group
@@ -224,7 +277,9 @@ __global__ void __launch_bounds__(kResMaxThreads) k_resident(const RArgs a) {
   double* gbuf = reinterpret_cast<double*>(sc + a.nstr);   // chunk rows of T partial cross sums
   double* gsum = gbuf + (a.grad ? a.chunk * T : 0);        // four cross sums per group with gradients
   RGroup* groups = reinterpret_cast<RGroup*>(gsum + (a.grad ? 4 * a.ngrad : 0));
-  uint32_t* sz = reinterpret_cast<uint32_t*>(groups + a.ngroups);   // parity mask | constant << 31
+  RStage* stages = reinterpret_cast<RStage*>(groups + a.ngroups);
+  ROp* ops = reinterpret_cast<ROp*>(stages + a.nstages);
+  uint32_t* sz = reinterpret_cast<uint32_t*>(ops + a.nops);   // parity mask | constant << 31
   uint32_t* fv = sz + a.nstr;                              // flip masks, first strings
   int* fs = reinterpret_cast<int*>(fv + a.nflips);
   __shared__ double2 wsum[kResMaxThreads / 32];
@@ -234,12 +289,16 @@ __global__ void __launch_bounds__(kResMaxThreads) k_resident(const RArgs a) {
   for (int p = tx; p < dim; p += T) psi[rswz(p)] = init[p];
   for (int i = tx; i < a.ncs; i += T) {
     const RAngle ang = a.angles[i];
-    const double t = ang.slot >= 0 ? a.theta[ang.slot] : ang.value;
+    const double t = ang.slot < 0 ? ang.value : a.theta ? a.theta[ang.slot] : th.v[ang.slot];
     double s, c;
     sincos(ang.family == MB_FAM_PHASE ? t : 0.5 * t, &s, &c);
     cs[i] = make_double2(c, s);
   }
   for (int i = tx; i < a.nmat; i += T) mat[i] = a.table[a.mat_off[i]];
+  for (int i = tx; i < a.nstages; i += T) stages[i] = a.stages[i];
+  for (int i = tx; i < a.ngroups; i += T) groups[i] = a.groups[i];
+  for (int i = tx; i < a.nops; i += T) ops[i] = a.ops[i];
+  bool imag = false;                                       // some string coefficient is not real
   for (int i = tx; i < a.nstr; i += T) {
     const PString p = a.strings[i];
     uint32_t m = 0, k = 0;
@@ -247,6 +306,7 @@ __global__ void __launch_bounds__(kResMaxThreads) k_resident(const RArgs a) {
       if ((p.z >> t) & 1) m ^= a.row[t], k ^= (a.rconst >> t) & 1u;
     sz[i] = m | (k << 31);
     sc[i] = p.c;
+    imag |= p.c.y != 0.0;
   }
   for (int i = tx; i < a.nflips; i += T) {
     const PFlip f = a.flips[i];
@@ -257,63 +317,111 @@ __global__ void __launch_bounds__(kResMaxThreads) k_resident(const RArgs a) {
     fs[i] = f.s0;
     if (i + 1 == a.nflips) fs[i + 1] = f.s0 + f.ns;
   }
-  __syncthreads();
-  for (int i = tx; i < a.ngroups; i += T) {
-    const RGroup g = a.groups[i];
-    groups[i] = g;
-    if (g.kind != RG_PAIR) continue;
-    const M2 first = op_matrix(a.ops[g.op0], cs, a.table);
-    M2DD m{wide(first.m00), wide(first.m10), wide(first.m01), wide(first.m11)};
-    for (int o = 1; o < g.nops; ++o) m = mul(op_matrix(a.ops[g.op0 + o], cs, a.table), m);
-    gm[i] = M2{narrow(m.m00), narrow(m.m10), narrow(m.m01), narrow(m.m11)};
+  imag = __syncthreads_or(imag);
+  // two threads per group, one column each
+  for (int i = tx; i < 2 * a.ngroups; i += T) {
+    const RGroup g = groups[i >> 1];
+    const M2 first = op_matrix(ops[g.op0], cs, a.table);
+    CDD x = wide(i & 1 ? first.m01 : first.m00), y = wide(i & 1 ? first.m11 : first.m10);
+    for (int o = 1; o < g.nops; ++o) {
+      const M2 m = op_matrix(ops[g.op0 + o], cs, a.table);
+      const CDD u = x;
+      x = cdot(m.m00, u, m.m01, y);
+      y = cdot(m.m10, u, m.m11, y);
+    }
+    double2* out = reinterpret_cast<double2*>(gm + (i >> 1)) + 2 * (i & 1);   // m00, m10, m01, m11
+    out[0] = narrow(x);
+    out[1] = narrow(y);
   }
   __syncthreads();
 
+  const int nt = dim >> R;
+  const bool mine = tx < nt;
+  // Storage slots of this thread's tuple: local index m at at ^ (the flips of m's bits).
+  auto slots = [&](const RStage& g, int* sv, unsigned* base) {
+    int p = tx;
+#pragma unroll
+    for (int i = 0; i < R; ++i) p = insert0(p, g.pivot[i]);
+    int at = rswz(p);
+    unsigned q = unsigned(p);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      sv[i] = rswz(g.v[i]);
+      if (par(g.r[i] & unsigned(p)) ^ ((g.rc >> i) & 1u)) at ^= sv[i], q ^= g.v[i];
+    }
+    *base = q;
+    return at;
+  };
+  auto slot = [](int at, const int* sv, int m) {
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      if ((m >> i) & 1) at ^= sv[i];
+    return at;
+  };
+
   // Forward.
-  for (int gi = 0; gi < a.ngroups; ++gi) {
-    const RGroup g = groups[gi];
-    if (g.kind != RG_PAIR) {
-      other_group(g, mat, psi, n, false);
+  for (int si = 0; si < a.nstages; ++si) {
+    const RStage st = stages[si];
+    if (st.kind != RG_PAIRS) {
+      other_stage(st, mat, psi, n, false);
       __syncthreads();
       continue;
     }
-    const M2 m = gm[gi];
-    const int sv = rswz(g.v);
-    // every pair is loaded before one is stored: the loads of a thread overlap
-    int i0[PAIRS];
-    double2 x[PAIRS], y[PAIRS];
+    if (mine) {
+      int sv[R];
+      unsigned base;
+      const int at = slots(st, sv, &base);
+      double2 x[A];
 #pragma unroll
-    for (int k = 0; k < PAIRS; ++k) {
-      const int p = insert0(tx + k * T, g.pivot);
-      i0[k] = tx + k * T < npairs && controls_on(g, p) ? rswz(p) ^ ((par(g.r & p) ^ g.rc) ? sv : 0) : -1;
-      if (i0[k] >= 0) x[k] = psi[i0[k]], y[k] = psi[i0[k] ^ sv];
-    }
-#pragma unroll
-    for (int k = 0; k < PAIRS; ++k)
-      if (i0[k] >= 0) {
-        apply(m, x[k], y[k]);
-        psi[i0[k]] = x[k];
-        psi[i0[k] ^ sv] = y[k];
+      for (int m = 0; m < A; ++m) x[m] = psi[slot(at, sv, m)];
+      for (int gi = st.g0; gi < st.g0 + st.ng; ++gi) {
+        const RGroup& g = groups[gi];
+        const M2 m = gm[gi];
+        if (g.nctl == 0) {
+          on_bit<R>(g.bit, [&](auto k) { apply_bit<R, decltype(k)::value, true>(x, m, 0u); });
+        } else {
+          const unsigned on = pairs_on<R>(g, base);
+          on_bit<R>(g.bit, [&](auto k) { apply_bit<R, decltype(k)::value, false>(x, m, on); });
+        }
       }
+#pragma unroll
+      for (int m = 0; m < A; ++m) psi[slot(at, sv, m)] = x[m];
+    }
     __syncthreads();
   }
 
   // <H>, and delta = 2 H psi for the reverse (Hermitian H, expectation.jl:4-73).
+  // A thread takes its 2^R amplitudes together, so a string is read once for all of them.
   double2 e = cz();
-  for (int p = tx; p < dim; p += T) {
-    double2 h = cz();
+  if (mine) {
+    double2 h[A];
+#pragma unroll
+    for (int k = 0; k < A; ++k) h[k] = cz();
     for (int f = 0; f < a.nflips; ++f) {
-      const unsigned src = unsigned(p) ^ fv[f];
-      double2 c = cz();
+      const unsigned x = fv[f];
+      double2 c[A];
+#pragma unroll
+      for (int k = 0; k < A; ++k) c[k] = cz();
       for (int s = fs[f]; s < fs[f + 1]; ++s) {
-        const bool odd = (par(sz[s] & 0x7fffffffu & src) ^ (sz[s] >> 31)) != 0;
-        c.x += odd ? -sc[s].x : sc[s].x;
-        c.y += odd ? -sc[s].y : sc[s].y;
+        const uint32_t z = sz[s];
+        const double2 v = sc[s];
+#pragma unroll
+        for (int k = 0; k < A; ++k) {
+          const unsigned src = unsigned(tx + k * nt) ^ x;
+          const long long flip = (long long)(par(z & 0x7fffffffu & src) ^ (z >> 31)) << 63;
+          c[k].x += __longlong_as_double(__double_as_longlong(v.x) ^ flip);
+          if (imag) c[k].y += __longlong_as_double(__double_as_longlong(v.y) ^ flip);
+        }
       }
-      h = cfma(c, psi[rswz(int(src))], h);
+#pragma unroll
+      for (int k = 0; k < A; ++k) h[k] = cfma(c[k], psi[rswz((tx + k * nt) ^ int(x))], h[k]);
     }
-    e = cfma_conj(psi[rswz(p)], h, e);
-    if (a.grad) del[rswz(p)] = make_double2(2.0 * h.x, 2.0 * h.y);
+#pragma unroll
+    for (int k = 0; k < A; ++k) {
+      const int i = rswz(tx + k * nt);
+      e = cfma_conj(psi[i], h[k], e);
+      if (a.grad) del[i] = make_double2(2.0 * h[k].x, 2.0 * h[k].y);
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -344,60 +452,70 @@ __global__ void __launch_bounds__(kResMaxThreads) k_resident(const RArgs a) {
     done += row;
     row = 0;
   };
-  for (int gi = a.ngroups - 1; gi >= 0; --gi) {
-    const RGroup g = groups[gi];
-    if (g.kind != RG_PAIR) {
-      other_group(g, mat, psi, n, true);
-      other_group(g, mat, del, n, true);
+  for (int si = a.nstages - 1; si >= 0; --si) {
+    const RStage st = stages[si];
+    if (st.kind != RG_PAIRS) {
+      other_stage(st, mat, psi, n, true);
+      other_stage(st, mat, del, n, true);
       __syncthreads();
       continue;
     }
-    const M2 m = dagger(gm[gi]);
-    const int sv = rswz(g.v);
-    const bool want = g.grad >= 0;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-    int i0[PAIRS];
-    double2 x[PAIRS], y[PAIRS], dx[PAIRS], dy[PAIRS];
+    int sv[R], at = 0;
+    unsigned base = 0;
+    double2 y[A], d[A];
+    if (mine) {
+      at = slots(st, sv, &base);
 #pragma unroll
-    for (int k = 0; k < PAIRS; ++k) {
-      const int p = insert0(tx + k * T, g.pivot);
-      i0[k] = tx + k * T < npairs && controls_on(g, p) ? rswz(p) ^ ((par(g.r & p) ^ g.rc) ? sv : 0) : -1;
-      if (i0[k] >= 0) {
-        x[k] = psi[i0[k]];
-        y[k] = psi[i0[k] ^ sv];
-        dx[k] = del[i0[k]];
-        dy[k] = del[i0[k] ^ sv];
+      for (int m = 0; m < A; ++m) {
+        const int i = slot(at, sv, m);
+        y[m] = psi[i];
+        d[m] = del[i];
       }
     }
-#pragma unroll
-    for (int k = 0; k < PAIRS; ++k)
-      if (i0[k] >= 0) {
-        if (want) {
-          s0 = fma(dx[k].y, x[k].x, fma(-dx[k].x, x[k].y, s0));
-          s1 = fma(dy[k].y, y[k].x, fma(-dy[k].x, y[k].y, s1));
-          s2 = fma(dx[k].y, y[k].x, fma(-dx[k].x, y[k].y, fma(dy[k].y, x[k].x, fma(-dy[k].x, x[k].y, s2))));
-          s3 = fma(dx[k].x, y[k].x, fma(dx[k].y, y[k].y, fma(-dy[k].x, x[k].x, fma(-dy[k].y, x[k].y, s3))));
+    for (int gi = st.g0 + st.ng - 1; gi >= st.g0; --gi) {
+      const RGroup& g = groups[gi];
+      double s[4] = {0.0, 0.0, 0.0, 0.0};
+      if (mine) {
+        const M2 m = dagger(gm[gi]);
+        if (g.nctl == 0) {
+          on_bit<R>(g.bit, [&](auto k) {
+            constexpr int K = decltype(k)::value;
+            if (g.grad >= 0) cross_bit<R, K, true>(y, d, 0u, s);
+            apply_bit<R, K, true>(y, m, 0u);
+            apply_bit<R, K, true>(d, m, 0u);
+          });
+        } else {
+          const unsigned on = pairs_on<R>(g, base);
+          on_bit<R>(g.bit, [&](auto k) {
+            constexpr int K = decltype(k)::value;
+            if (g.grad >= 0) cross_bit<R, K, false>(y, d, on, s);
+            apply_bit<R, K, false>(y, m, on);
+            apply_bit<R, K, false>(d, m, on);
+          });
         }
-        apply(m, x[k], y[k]);
-        apply(m, dx[k], dy[k]);
-        psi[i0[k]] = x[k];
-        psi[i0[k] ^ sv] = y[k];
-        del[i0[k]] = dx[k];
-        del[i0[k] ^ sv] = dy[k];
       }
-    if (want) {
-      // lane bits 0 and 1 choose the sum a lane keeps
-      const bool b0 = tx & 1, b1 = tx & 2;
-      const double u0 = (b0 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, b0 ? s0 : s1, 1);
-      const double u1 = (b0 ? s3 : s2) + __shfl_xor_sync(0xffffffffu, b0 ? s2 : s3, 1);
-      gbuf[row * T + tx] = (b1 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, b1 ? u0 : u1, 2);
-      ++row;
+      if (g.grad >= 0) {
+        if (row == a.chunk) {
+          __syncthreads();
+          add_rows();
+          __syncthreads();
+        }
+        // lane bits 0 and 1 choose the sum a lane keeps
+        const bool b0 = tx & 1, b1 = tx & 2;
+        const double u0 = (b0 ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, b0 ? s[0] : s[1], 1);
+        const double u1 = (b0 ? s[3] : s[2]) + __shfl_xor_sync(0xffffffffu, b0 ? s[2] : s[3], 1);
+        gbuf[row * T + tx] = (b1 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, b1 ? u0 : u1, 2);
+        ++row;
+      }
     }
+    if (mine)
+#pragma unroll
+      for (int m = 0; m < A; ++m) {
+        const int i = slot(at, sv, m);
+        psi[i] = y[m];
+        del[i] = d[m];
+      }
     __syncthreads();
-    if (row == a.chunk) {
-      add_rows();
-      __syncthreads();
-    }
   }
   add_rows();
 
@@ -406,10 +524,10 @@ __global__ void __launch_bounds__(kResMaxThreads) k_resident(const RArgs a) {
   __syncthreads();
   const double scale = a.B > 1 ? 1.0 : a.weights[0];
   auto gate_gradient = [&](int o) {
-    const ROp op = a.ops[o];
+    const ROp op = ops[o];
     const RGroup g = groups[op.group];
-    M2 V = dagger(op_matrix(a.ops[g.op0 + g.nops - 1], cs, a.table));
-    for (int k = g.op0 + g.nops - 2; k >= o; --k) V = mul(dagger(op_matrix(a.ops[k], cs, a.table)), V);
+    M2 V = dagger(op_matrix(ops[g.op0 + g.nops - 1], cs, a.table));
+    for (int k = g.op0 + g.nops - 2; k >= o; --k) V = mul(dagger(op_matrix(ops[k], cs, a.table)), V);
     // generators (i/2)X, (i/2)Y, (i/2)Z, diag(0, -i)
     const double2 z = cz();
     M2 D{z, z, z, z};
@@ -424,12 +542,12 @@ __global__ void __launch_bounds__(kResMaxThreads) k_resident(const RArgs a) {
   };
   if (a.unique) {
     for (int o = tx; o < a.nops; o += T) {
-      const int slot = a.ops[o].slot;
+      const int slot = ops[o].slot;
       if (slot >= 0) gs[slot] = gate_gradient(o);
     }
   } else if (tx == 0) {
     for (int o = 0; o < a.nops; ++o) {
-      const int slot = a.ops[o].slot;
+      const int slot = ops[o].slot;
       if (slot >= 0) gs[slot] += gate_gradient(o);
     }
   }
@@ -454,45 +572,98 @@ __global__ void __launch_bounds__(kResMaxThreads) k_resident(const RArgs a) {
 struct Builder {
   mb_circuit c;
   ResidentPlan* P;
+  int R;
+  std::vector<RStage> stages;
   std::vector<RGroup> groups;
   std::vector<ROp> ops;
   std::vector<RAngle> angles;
   std::vector<int> mats;
+  struct Control {
+    uint16_t n = 0, ctl[4] = {0, 0, 0, 0}, cbits = 0;
+  };
   struct Held {
     ROp op;
-    RGroup ctl;   // its controls
+    Control ctl;
   };
   std::vector<Held> open[kResMaxBits];
   uint16_t row[kResMaxBits], col[kResMaxBits], rconst = 0;
+  // The stage being filled: its targets and the frame it runs in.
+  bool filling = false;
+  std::vector<int> targets;
+  uint16_t srow[kResMaxBits], scol[kResMaxBits], sconst = 0;
 
   uint16_t bit(int t) const { return uint16_t((rconst >> t) & 1); }
   static uint16_t high_bit(unsigned v) { return uint16_t(31 - __builtin_clz(v)); }
 
-  RGroup target(int q) const {
-    RGroup g{};
-    g.v = col[q];
-    g.r = row[q];
-    g.rc = bit(q);
-    g.pivot = high_bit(col[q]);
-    return g;
+  // Pivots of `count` independent flip masks: storage bits of which every tuple has exactly one
+  // member with all of them clear.
+  static void pivots(const uint16_t* v, int count, uint16_t* out) {
+    uint16_t w[3];
+    for (int i = 0; i < count; ++i) {
+      w[i] = v[i];
+      for (int j = 0; j < i; ++j)
+        if ((w[i] >> out[j]) & 1) w[i] ^= w[j];
+      out[i] = high_bit(w[i]);
+      for (int j = 0; j < i; ++j)
+        if ((w[j] >> out[i]) & 1) w[j] ^= w[i];
+    }
+    std::sort(out, out + count);
+  }
+  void finish_stage() {
+    if (!filling) return;
+    filling = false;
+    RStage& s = stages.back();
+    // free places hold other qubits of the frame
+    for (int q = 0; q < c->n && int(targets.size()) < R; ++q)
+      if (std::find(targets.begin(), targets.end(), q) == targets.end()) targets.push_back(q);
+    for (int i = 0; i < R; ++i) {
+      s.v[i] = scol[targets[i]];
+      s.r[i] = srow[targets[i]];
+      s.rc |= uint16_t(((sconst >> targets[i]) & 1) << i);
+    }
+    pivots(s.v, R, s.pivot);
+    for (int g = s.g0; g < s.g0 + s.ng; ++g)
+      for (int k = 0; k < groups[g].nctl; ++k)
+        for (int i = 0; i < R; ++i)
+          groups[g].cm |= uint16_t((__builtin_popcount(groups[g].ctl[k] & s.v[i]) & 1) << (4 * k + i));
+  }
+  // Local bit of qubit q in the stage being filled, starting another if q or its frame does not fit.
+  int place(int q) {
+    if (filling && (scol[q] != col[q] || srow[q] != row[q] || ((sconst >> q) & 1) != bit(q))) finish_stage();
+    if (filling) {
+      const auto it = std::find(targets.begin(), targets.end(), q);
+      if (it != targets.end()) return int(it - targets.begin());
+      if (int(targets.size()) == R) finish_stage();
+    }
+    if (!filling) {
+      filling = true;
+      targets.clear();
+      std::copy(row, row + c->n, srow);
+      std::copy(col, col + c->n, scol);
+      sconst = rconst;
+      RStage s{};
+      s.kind = RG_PAIRS;
+      s.g0 = uint16_t(groups.size());
+      stages.push_back(s);
+    }
+    targets.push_back(q);
+    return int(targets.size()) - 1;
   }
   void close(int q) {
     if (open[q].empty()) return;
-    RGroup g = target(q);
-    const RGroup& last = open[q].back().ctl;
     // a controlled gate is a group by itself: its predecessors on the target go before it
-    const size_t count = open[q].size() - (last.nctl ? 1 : 0);
-    if (count) emit(g, open[q].data(), count);
-    if (last.nctl) {
-      g.nctl = last.nctl;
-      std::memcpy(g.ctl, last.ctl, sizeof(g.ctl));
-      g.cbits = last.cbits;
-      emit(g, &open[q].back(), 1);
-    }
+    const Control& last = open[q].back().ctl;
+    const size_t count = open[q].size() - (last.n ? 1 : 0);
+    if (count) emit(q, Control(), open[q].data(), count);
+    if (last.n) emit(q, last, &open[q].back(), 1);
     open[q].clear();
   }
-  void emit(RGroup g, const Held* h, size_t count) {
-    g.kind = RG_PAIR;
+  void emit(int q, const Control& ctl, const Held* h, size_t count) {
+    RGroup g{};
+    g.bit = uint16_t(place(q));
+    g.nctl = ctl.n;
+    std::copy(ctl.ctl, ctl.ctl + 4, g.ctl);
+    g.cbits = ctl.cbits;
     g.op0 = uint16_t(ops.size());
     g.nops = uint16_t(count);
     g.grad = -1;
@@ -502,21 +673,22 @@ struct Builder {
       if (h[i].op.slot >= 0) g.grad = 0;
     }
     groups.push_back(g);
+    stages.back().ng += 1;
   }
-  void controls(RGroup& g, const int* q, int count) {
-    g.nctl = uint16_t(count);
+  Control controls(const int* q, int count) const {
+    Control k;
+    k.n = uint16_t(count);
     for (int j = 0; j < count; ++j) {
-      g.ctl[j] = row[q[j]];
-      g.cbits |= uint16_t(bit(q[j]) << j);
+      k.ctl[j] = row[q[j]];
+      k.cbits |= uint16_t(bit(q[j]) << j);
     }
+    return k;
   }
   // A single-target gate: it joins the target's open group; with controls it also ends it, so that
   // later gates on a control cannot be emitted before it.
   void single(ROp op, int t, const int* ctl, int nctl) {
     for (int j = 0; j < nctl; ++j) close(ctl[j]);
-    Held h{op, RGroup{}};
-    controls(h.ctl, ctl, nctl);
-    open[t].push_back(h);
+    open[t].push_back(Held{op, controls(ctl, nctl)});
     if (nctl) close(t);
   }
   uint16_t matrix(const COp& o, int count, const int* elems) {
@@ -596,38 +768,46 @@ struct Builder {
       return true;
     }
     for (int j = 0; j < o.k; ++j) close(o.pos[j]);
-    RGroup g = target(o.pos[0]);
-    g.grad = -1;
+    RStage g{};
+    g.v[0] = col[o.pos[0]];
+    g.r[0] = row[o.pos[0]];
+    g.rc = bit(o.pos[0]);
     if (o.cls == CLS_DIAG) {
       g.kind = RG_DIAG;
       int e[32];
       for (int i = 0; i < d; ++i) e[i] = i * (d + 1);
-      g.op0 = matrix(o, d, e);
-      controls(g, o.pos + 1, o.k - 1);
+      g.g0 = matrix(o, d, e);
+      const Control k = controls(o.pos + 1, o.k - 1);
+      g.nctl = k.n;
+      std::copy(k.ctl, k.ctl + 4, g.ctl);
+      g.cbits = k.cbits;
     } else if (o.k == 2) {
       g.kind = RG_U2;
       int e[16];
       for (int i = 0; i < 16; ++i) e[i] = i;
-      g.op0 = matrix(o, 16, e);
-      const int q = o.pos[1];
-      g.v2 = col[q];
-      g.r2 = row[q];
-      g.rc2 = bit(q);
-      const unsigned w = ((g.v2 >> g.pivot) & 1) ? g.v2 ^ g.v : g.v2;   // v2 without the first pivot
-      g.pivot2 = high_bit(w);
+      g.g0 = matrix(o, 16, e);
+      g.v[1] = col[o.pos[1]];
+      g.r[1] = row[o.pos[1]];
+      g.rc |= uint16_t(bit(o.pos[1]) << 1);
+      pivots(g.v, 2, g.pivot);
     } else {
       return false;
     }
-    groups.push_back(g);
+    finish_stage();
+    stages.push_back(g);
     return true;
   }
 };
+
+// Qubits per stage: three from 9 qubits; below, two keep more than one warp busy (8 qubits: 64 threads).
+int resident_width(int n) { return n >= 9 ? 3 : n >= 4 ? 2 : 1; }
+int resident_threads(int n) { return std::max(32, 1 << (n - resident_width(n))); }
 
 size_t resident_shared(const ResidentPlan& P, int nflips, int nstr, bool grad, int T, int chunk) {
   size_t s = (sizeof(double2) << P.n) * (grad ? 2 : 1);
   s += sizeof(double2) * (size_t(P.ncs) + P.nmat + nstr) + sizeof(M2) * size_t(P.ngroups);
   if (grad) s += sizeof(double) * (size_t(chunk) * T + 4 * size_t(P.ngrad));
-  s += sizeof(RGroup) * size_t(P.ngroups);
+  s += sizeof(RGroup) * size_t(P.ngroups) + sizeof(RStage) * size_t(P.nstages) + sizeof(ROp) * size_t(P.nops);
   s += sizeof(uint32_t) * (size_t(nstr) + 2 * size_t(nflips) + 1);
   return (s + 15) & ~size_t(15);
 }
@@ -637,6 +817,7 @@ int build_plan(mb_circuit c, ResidentPlan* P) {
   Builder B;
   B.c = c;
   B.P = P;
+  B.R = resident_width(c->n);
   for (int t = 0; t < c->n; ++t) B.row[t] = B.col[t] = uint16_t(1 << t);
   for (const COp& o : c->ops) {
     // 16-bit indexes, and room left in shared memory in any case
@@ -644,6 +825,7 @@ int build_plan(mb_circuit c, ResidentPlan* P) {
     if (!B.add(o)) return MB_OK;
   }
   for (int q = 0; q < c->n; ++q) B.close(q);
+  B.finish_stage();
   // rows of the cross sums in the order the reverse meets the groups
   for (size_t g = B.groups.size(); g-- > 0;)
     if (B.groups[g].grad >= 0) {
@@ -656,6 +838,7 @@ int build_plan(mb_circuit c, ResidentPlan* P) {
       P->unique = P->unique && !seen[op.slot];
       seen[op.slot] = 1;
     }
+  P->nstages = int(B.stages.size());
   P->ngroups = int(B.groups.size());
   P->nops = int(B.ops.size());
   P->ncs = int(B.angles.size());
@@ -670,7 +853,8 @@ int build_plan(mb_circuit c, ResidentPlan* P) {
     if (bytes) std::memcpy(h.data() + at, d, bytes);
     return at;
   };
-  put(B.groups.data(), sizeof(RGroup) * B.groups.size());
+  put(B.stages.data(), sizeof(RStage) * B.stages.size());
+  P->off_groups = put(B.groups.data(), sizeof(RGroup) * B.groups.size());
   P->off_ops = put(B.ops.data(), sizeof(ROp) * B.ops.size());
   P->off_ang = put(B.angles.data(), sizeof(RAngle) * B.angles.size());
   P->off_mat = put(B.mats.data(), sizeof(int) * B.mats.size());
@@ -680,8 +864,6 @@ int build_plan(mb_circuit c, ResidentPlan* P) {
   P->ok = true;
   return MB_OK;
 }
-
-int resident_threads(int n) { return n <= 6 ? 32 : n <= 10 ? 1 << (n - 1) : kResMaxThreads; }
 
 }  // namespace
 
@@ -710,28 +892,32 @@ int resident_run(mb_circuit c, mb_observable o, mb_state init, const double* the
   const ResidentPlan& P = *c->resident;
   if (!P.ok) return MB_OK;
   const int T = resident_threads(n);
-  const int pairs = std::max(1, (1 << (n - 1)) / T);
   // Rows per chunk: 32 KiB of partial cross sums.
   const int chunk = std::max(4, 4096 / T);
   const size_t shm = resident_shared(P, os.nflips, os.nstr, grad != nullptr, T, chunk);
   if (shm > kResMaxShared) return MB_OK;
 
-  // Parameters and weights go up and results come back in one copy each, through pinned memory;
-  // the call waits for its results, so the buffers are free again when it returns.
-  const size_t up = size_t(c->nslots) + (grad ? size_t(B) : 0);
-  const size_t down = 2 * size_t(B) + (grad ? size_t(c->nslots) : 0);
-  const size_t rows = grad && B > 1 ? size_t(B) * c->nslots : 0;
-  if (int rc = small_reserve(up + down, up + down + rows)) return rc;
+  // Parameters travel with the launch and results are written to pinned memory: at these sizes each
+  // copy on the stream costs more than it moves. Weights, which only the last of several samples
+  // reads, and long parameter lists go up in a copy. The call waits for its results, so the buffers
+  // are free again when it returns.
+  const size_t ns = size_t(c->nslots), nw = grad ? size_t(B) : 0;
+  const size_t down = 2 * size_t(B) + (grad ? ns : 0), rows = grad && B > 1 ? size_t(B) * ns : 0;
+  if (int rc = small_reserve(ns + nw + down, ns + nw + rows)) return rc;
   double* hp = g_ctx.h_small;
   double* dp = g_ctx.d_small;
-  std::copy(theta, theta + c->nslots, hp);
-  if (grad) std::copy(weights, weights + B, hp + c->nslots);
+  RTheta th;
+  const bool direct = ns <= kResTheta;
+  std::copy(theta, theta + ns, direct ? th.v : hp);
+  if (grad) std::copy(weights, weights + B, hp + ns);
   cudaStream_t st = g_ctx.stream;
-  if (up) MB_CHECK_CUDA(cudaMemcpyAsync(dp, hp, sizeof(double) * up, cudaMemcpyHostToDevice, st));
+  const size_t first = direct ? ns : 0, up = B > 1 || !direct ? ns + nw - first : 0;
+  if (up) MB_CHECK_CUDA(cudaMemcpyAsync(dp + first, hp + first, sizeof(double) * up, cudaMemcpyHostToDevice, st));
 
   RArgs a{};
   a.n = n;
   a.grad = grad ? 1 : 0;
+  a.nstages = P.nstages;
   a.ngroups = P.ngroups;
   a.nops = P.nops;
   a.ncs = P.ncs;
@@ -747,37 +933,36 @@ int resident_run(mb_circuit c, mb_observable o, mb_state init, const double* the
   std::memcpy(a.col, P.col, sizeof(a.col));
   a.rconst = P.rconst;
   const unsigned char* d = static_cast<const unsigned char*>(P.d);
-  a.groups = reinterpret_cast<const RGroup*>(d);
+  a.stages = reinterpret_cast<const RStage*>(d);
+  a.groups = reinterpret_cast<const RGroup*>(d + P.off_groups);
   a.ops = reinterpret_cast<const ROp*>(d + P.off_ops);
   a.angles = reinterpret_cast<const RAngle*>(d + P.off_ang);
   a.mat_off = reinterpret_cast<const int*>(d + P.off_mat);
   a.table = c->d_table;
-  a.theta = dp;
-  a.weights = dp + c->nslots;
+  a.theta = direct ? nullptr : dp;
+  a.weights = (B > 1 ? dp : hp) + ns;
   a.init = init->d;
   a.flips = os.flips;
   a.strings = os.strings;
-  double* res = dp + up;
-  a.values = reinterpret_cast<double2*>(res + (up & 1));   // 16-byte aligned; small_reserve leaves room
-  a.gout = reinterpret_cast<double*>(a.values + B);
-  a.gsample = a.gout + c->nslots;
+  double* res = hp + ns + nw + ((ns + nw) & 1);   // 16-byte aligned; small_reserve leaves room
+  a.values = reinterpret_cast<double2*>(res);
+  a.gout = res + 2 * size_t(B);
+  a.gsample = dp + ns + nw;
   a.counter = g_ctx.counters;
   auto launch = [&](auto kern) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm));
-    kern<<<B, T, shm, st>>>(a);
+    kern<<<B, T, shm, st>>>(a, th);
   };
   {
     ProfScope ps("k_resident", 16.0 * double(init->elems) * B, st);
-    if (pairs == 1) launch(k_resident<1>);
-    else if (pairs == 2) launch(k_resident<2>);
-    else launch(k_resident<4>);
+    if (resident_width(n) == 3) launch(k_resident<3>);
+    else if (resident_width(n) == 2) launch(k_resident<2>);
+    else launch(k_resident<1>);
   }
   MB_LAUNCHED();
-  double* hr = hp + up;
-  MB_CHECK_CUDA(cudaMemcpyAsync(hr, a.values, sizeof(double) * down, cudaMemcpyDeviceToHost, st));
   MB_CHECK_CUDA(cudaStreamSynchronize(st));
-  std::memcpy(values, hr, sizeof(double2) * B);
-  if (grad) std::copy(hr + 2 * size_t(B), hr + down, grad);
+  std::memcpy(values, res, sizeof(double2) * B);
+  if (grad) std::copy(res + 2 * size_t(B), res + down, grad);
   *done = true;
   return MB_OK;
 }
