@@ -164,19 +164,78 @@ __global__ void __launch_bounds__(128) k_reg_pass(double2* __restrict__ v, const
   }
 }
 
+// One record's product by G lanes (4 for 2x2 products, 16 for 4x4): lane r + d c of the group holds
+// entry (r, c); every component is read by the lanes that hold its entries (a 2x2 inside a 4x4
+// widened by zeros) and multiplied through shuffles. Bound by the latency of a component's two
+// dependent reads (offset, entry), so four components are read together: 40 records of up to 16
+// components (density matrix of 10 qubits) took 45 us with one thread per record, now 19. All lanes of
+// the warp enter (a lane without a record passes nc = 0): groups run to the longest record of the warp.
+template <int G>
+__device__ __forceinline__ void fuse_record(const FuseRec& r, int nc, const FuseComp* __restrict__ comps,
+                                            const double2* __restrict__ row0, const double2* __restrict__ rowb,
+                                            double2* out) {
+  const int lane = threadIdx.x & (G - 1);
+  constexpr int d = G == 16 ? 4 : 2;
+  const int row = lane & (d - 1), col = lane / d;
+  double2 M = make_double2(row == col ? 1.0 : 0.0, 0.0);
+  auto entry = [&](int ci) {
+    const FuseComp* c = comps + r.c0 + ci;
+    const int kind = c->kind;
+    int e = row + d * col;
+    if (kind != FC_DENSE4) {
+      const int bit = d == 4 ? c->bit : 0, other = 1 ^ bit;
+      if (d == 4 && ((row ^ col) >> other) & 1) return cz();
+      const int rb = (row >> bit) & 1, cb = (col >> bit) & 1;
+      if (kind == FC_DENSE2) {
+        e = rb + 2 * cb;
+      } else {
+        if (rb != cb) return cz();
+        if (kind == FC_PHASE2) {
+          if (rb == 0) return make_double2(1.0, 0.0);
+          if (c->neg) return make_double2(-1.0, 0.0);
+          e = 0;
+        } else {
+          if (!((c->active >> rb) & 1)) return make_double2(1.0, 0.0);
+          e = rb;
+        }
+      }
+    }
+    const double2 v = (c->param ? rowb : row0)[c->off[e]];
+    return c->conj ? make_double2(v.x, -v.y) : v;
+  };
+  const int most = __reduce_max_sync(0xffffffffu, nc);
+  for (int c0 = 0; c0 < most; c0 += 4) {
+    double2 X[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) X[k] = c0 + k < nc ? entry(c0 + k) : cz();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      double2 acc = cz();
+#pragma unroll
+      for (int m = 0; m < d; ++m) {
+        const double2 x = make_double2(__shfl_sync(0xffffffffu, X[k].x, row + d * m, G),
+                                       __shfl_sync(0xffffffffu, X[k].y, row + d * m, G));
+        const double2 y = make_double2(__shfl_sync(0xffffffffu, M.x, m + d * col, G),
+                                       __shfl_sync(0xffffffffu, M.y, m + d * col, G));
+        acc = cfma(x, y, acc);
+      }
+      if (c0 + k < nc) M = acc;
+    }
+  }
+  if (nc > 0) out[r.out + lane] = M;
+}
+
 // Per-sample products of the fused single-qubit runs (after binding): row b of the derived
-// table's per-sample region gets every record's product formed from table row b.
-__global__ void k_fuse(const FuseRec* __restrict__ recs, int nrecs, const FuseComp* __restrict__ comps,
-                       const double2* __restrict__ table, int64_t tstride, double2* __restrict__ xs, int64_t xrow,
-                       int rows) {
-  const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (idx >= int64_t(nrecs) * rows) return;
-  const int b = int(idx / nrecs);
-  const FuseRec r = recs[idx % nrecs];
-  double2 M[16];
-  fuse_product(r, comps, table, table + int64_t(b) * tstride, M);
-  double2* out = xs + int64_t(b) * xrow + r.out;
-  for (int e = 0; e < r.d * r.d; ++e) out[e] = M[e];
+// table's per-sample region gets every record's product formed from table row b, G lanes each.
+template <int G>
+__global__ void __launch_bounds__(128) k_fuse(const FuseRec* __restrict__ recs, int nrecs,
+                                              const FuseComp* __restrict__ comps, const double2* __restrict__ table,
+                                              int64_t tstride, double2* __restrict__ xs, int64_t xrow, int rows) {
+  const int64_t total = int64_t(nrecs) * rows;
+  const int64_t w = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / G, idx = w < total ? w : total - 1;
+  const int64_t b = idx / nrecs;
+  const FuseRec& r = recs[idx % nrecs];
+  fuse_record<G>(r, w < total ? r.nc : 0, comps, table, table + b * tstride, xs + b * xrow);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -245,17 +304,12 @@ __global__ void k_uneven_bind(const UnevenGroup* __restrict__ groups, int ng, in
 }
 
 // Fused single-qubit products of every sample of every group: item = (group, sample, record).
-__global__ void k_uneven_fuse(const UnevenGroup* __restrict__ groups, int ng, int64_t total) {
-  const int64_t w = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (w >= total) return;
-  const UnevenGroup& G = groups[uneven_group_of(groups, ng, w, true)];
-  const int64_t r = w - G.fuse0;
-  const int b = int(r / G.nrecs), q = int(r % G.nrecs);
-  const FuseRec rec = G.recs[q];
-  double2 M[16];
-  fuse_product(rec, G.comps, G.table, G.table + int64_t(b) * G.tstride, M);
-  double2* out = G.xtabs + int64_t(b) * G.xrow + rec.out;
-  for (int e = 0; e < rec.d * rec.d; ++e) out[e] = M[e];
+__global__ void __launch_bounds__(128) k_uneven_fuse(const UnevenGroup* __restrict__ groups, int ng, int64_t total) {
+  const int64_t i = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 4, w = i < total ? i : total - 1;
+  const UnevenGroup& U = groups[uneven_group_of(groups, ng, w, true)];
+  const int64_t q = w - U.fuse0, b = q / U.nrecs;
+  const FuseRec& r = U.recs[q % U.nrecs];
+  fuse_record<4>(r, i < total ? r.nc : 0, U.comps, U.table, U.table + b * U.tstride, U.xtabs + b * U.xrow);
 }
 
 // Work item: x = group, y = sample, z = pass index within the group, w = chunk.
@@ -2308,6 +2362,16 @@ static void prepare_jit(Schedule* S) {
   if (!g_ctx.capturing) jit_trim();
 }
 
+static int launch_fuse(Schedule* S, const double2* table, int64_t tstride, double2* xs, int rows) {
+  const int nrecs = int(S->frecs.size()), per = S->frecs[0].d == 4 ? 8 : 32;
+  const unsigned grid = unsigned((int64_t(nrecs) * rows + per - 1) / per);
+  ProfScope ps("k_fuse", 0.0, g_ctx.stream);
+  auto* k = per == 8 ? k_fuse<16> : k_fuse<4>;
+  k<<<grid, 128, 0, g_ctx.stream>>>(S->d_frecs, nrecs, S->d_fcomps, table, tstride, xs, S->xrow, rows);
+  MB_LAUNCHED();
+  return MB_OK;
+}
+
 int run_schedule(mb_circuit c, Schedule* S, double2* v, int nsamples, int64_t mstride) {
   cudaStream_t st = g_ctx.stream;
   const int N = S->N;
@@ -2321,12 +2385,7 @@ int run_schedule(mb_circuit c, Schedule* S, double2* v, int nsamples, int64_t ms
   double2* xs = S->d_xtab ? S->d_xtab + S->xtab.size() : nullptr;
   const int64_t xrow = mstride ? S->xrow : 0;
   if (!S->frecs.empty()) {
-    const int rows = mstride ? nsamples : 1;
-    const int64_t work = int64_t(S->frecs.size()) * rows;
-    ProfScope ps("k_fuse", 0.0, st);
-    k_fuse<<<unsigned((work + 127) / 128), 128, 0, st>>>(S->d_frecs, int(S->frecs.size()), S->d_fcomps, c->d_table,
-                                                          mstride, xs, S->xrow, rows);
-    MB_LAUNCHED();
+    if (int rc = launch_fuse(S, c->d_table, mstride, xs, mstride ? nsamples : 1)) return rc;
   }
   for (const Pass& p : S->passes) {
     int rc = MB_OK;
@@ -2487,10 +2546,7 @@ int run_adjoint_schedule(mb_circuit c, Schedule* S, double2* y, double2* d, doub
   const int B = S->nsamples;
   double2* xs = S->d_xtab ? S->d_xtab + S->xtab.size() : nullptr;
   if (!S->frecs.empty()) {
-    ProfScope ps("k_fuse", 0.0, st);
-    k_fuse<<<unsigned((S->frecs.size() + 127) / 128), 128, 0, st>>>(S->d_frecs, int(S->frecs.size()), S->d_fcomps,
-                                                                     c->d_table, 0, xs, S->xrow, 1);
-    MB_LAUNCHED();
+    if ((rc = launch_fuse(S, c->d_table, 0, xs, 1))) return rc;
   }
   for (const Pass& p : S->passes) {
     if (p.kind == PASS_PLAIN) {
@@ -2892,7 +2948,7 @@ extern "C" int mb_uneven_apply(mb_uneven u, int flags) {
     }
     if (u->nfuse) {
       ProfScope ps("k_uneven_fuse", 0.0, st);
-      k_uneven_fuse<<<unsigned((u->nfuse + 127) / 128), 128, 0, st>>>(u->d_groups, ng, u->nfuse);
+      k_uneven_fuse<<<unsigned((u->nfuse + 31) / 32), 128, 0, st>>>(u->d_groups, ng, u->nfuse);
       MB_LAUNCHED();
     }
     MB_CHECK_CUDA(cudaMemsetAsync(u->d_next, 0, sizeof(unsigned) * (1 + size_t(u->nsamples)), st));
