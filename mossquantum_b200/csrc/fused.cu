@@ -2006,14 +2006,19 @@ static bool want_jit(int N) {
 // Defaults: sizes run by the specialised kernels use the shape below; the interpreter kernels
 // use 2^12 tiles with 16 amplitudes per thread. mb_tuning_set / the autotuner override both per
 // register size.
-static Tuning tuning_for(int N) {
+static Tuning tuning_for(int N, bool whole = true) {
   Tuning tu;
   if (want_jit(N) && jit_available()) {
-    // 2^10-amplitude tiles, 8 amplitudes per thread, 4 CTAs of 128 threads per SM: the fastest
-    // point of a sweep over (t, R, CTAs) on the 28-qubit U3 + CZ step (62.5 ms against 63.8 ms
-    // at 2^11 tiles with 2 CTAs of 256 threads, 67.7 ms at 2^12 with 1 CTA of 512)
+    // 2^10-amplitude tiles. The passes load the FP64 pipe and the shared-memory pipe alike (55 to
+    // 60 % of each), so 16 amplitudes per thread with 6 CTAs of 64 threads beat 8 amplitudes with 4
+    // CTAs of 128: fewer stages move the tile, half the warps read the matrices. 28-qubit U3 + CZ
+    // step 48.5 against 51.4 ms, 20 x 20 RX/RY/RZ + CNOT 405 against 425 us, noisy 11 qubits 562
+    // against 610. Below 2^20 amplitudes 64-thread CTAs leave the chip short of warps (18 qubits: 137
+    // against 122 us, noisy 9 qubits 102 against 96), and the short segments of a checkpointed
+    // gradient are mostly light passes (24 qubits: 6.50 against 6.36 ms). 32 amplitudes with
+    // 6 warps: no faster, compile times past the budget. 2^11 tiles: 5.62 against 5.43 ms (25 qubits).
     tu.t = 10;
-    tu.R = 3;
+    tu.R = N >= 20 && whole ? 4 : 3;
   }
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -2045,7 +2050,7 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
                              const Tuning* force, bool tile_only, Schedule** out) {
   const int N = dm ? 2 * n : n;
   if (hi < 0) hi = int(c->ops.size());
-  Tuning tu = tuning_for(N);
+  Tuning tu = tuning_for(N, lo == 0 && hi == int(c->ops.size()));
   if (force) {
     tu.t = std::min(force->t, N);
     tu.R = force->R;
@@ -2219,11 +2224,12 @@ int get_schedule(mb_circuit c, int n, int dm, bool dagger, int nsamples, Schedul
 
 // CTAs per SM of a specialised tile pass: as many double-buffered tiles as shared memory holds
 // (allowing 4 KB for the pass's matrix copy; a larger copy only lowers the resident count),
-// capped at MB_TILE_CTAS (default 4 for tiles of at most 2^10 amplitudes, else 2). The kernel's launch bounds ask the compiler to fit that
-// many CTAs in the register file.
-static int tile_ctas(int t) {
+// capped at MB_TILE_CTAS (default for tiles of at most 2^10 amplitudes: 16 warps, or 12 of 16 amplitudes
+// per thread; else 2). The kernel's launch bounds ask the compiler to fit that many CTAs in the
+// register file.
+static int tile_ctas(int t, int R) {
   const size_t shm = (size_t(32) << t) + 1024 + 4 * 1024;
-  int cap = t <= 10 ? 4 : 2;
+  int cap = t > 10 ? 2 : R == 4 ? 6 : 4;
   if (const char* e = getenv("MB_TILE_CTAS")) cap = std::max(1, std::min(8, atoi(e)));
   return std::max(1, std::min(cap, int((227 * 1024) / (shm + 256))));
 }
@@ -2310,7 +2316,7 @@ static void prepare_jit(Schedule* S) {
   // staged in shared memory with the fixed ones (reverse sweeps share the parameters in any case).
   const bool single = S->nsamples == 1;
   for (Pass& p : S->passes) {
-    if (p.kind == PASS_TILE && !S->adjoint) p.ctas = tile_ctas(p.t);
+    if (p.kind == PASS_TILE && !S->adjoint) p.ctas = tile_ctas(p.t, S->R);
     if (p.kind == PASS_TILE && S->adjoint) {
       p.ctas = adjoint_ctas(p.t, S->dm);
       src.push_back(memo_source(pass_key(p, 1, S->R, S->N, true, p.ctas),
@@ -3102,7 +3108,7 @@ extern "C" int mb_schedule_info(const mb_op* ops, size_t nops, int n, int dm, in
     int i = 0;
     for (mb::Pass& ps : S.passes) {
       std::string src;
-      if (ps.kind == mb::PASS_TILE) src = mb::jit_tile_source(ps, S.R, N, nsamples == 1, mb::tile_ctas(ps.t));
+      if (ps.kind == mb::PASS_TILE) src = mb::jit_tile_source(ps, S.R, N, nsamples == 1, mb::tile_ctas(ps.t, S.R));
       else if (ps.kind == mb::PASS_REG) src = mb::jit_reg_source(ps, N, nsamples == 1);
       else continue;
       char path[512];
