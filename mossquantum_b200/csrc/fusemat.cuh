@@ -88,4 +88,29 @@ __host__ __device__ inline void fuse_product(const FuseRec& r, const FuseComp* c
   }
 }
 
+// A run's product is rounded once: its entries are carried as high and low parts, because an error
+// of the matrix is the same for every amplitude and adds up over the steps, where roundings of
+// amplitudes average out.
+struct DD {
+  double h, l;
+};
+__device__ __forceinline__ DD dd_fma(double a, DD b, DD c) {
+  const double p = a * b.h, q = fma(a, b.h, -p) + a * b.l;     // a * b
+  const double s = c.h + p, z = s - c.h;
+  const double r = ((c.h - (s - z)) + (p - z)) + (c.l + q);    // two-sum of the high parts
+  const double h = s + r;
+  return DD{h, r - (h - s)};
+}
+struct CDD {
+  DD x, y;
+};
+__device__ __forceinline__ CDD wide(double2 a) { return CDD{DD{a.x, 0.0}, DD{a.y, 0.0}}; }
+__device__ __forceinline__ double2 narrow(const CDD& a) { return make_double2(a.x.h, a.y.h); }
+// a * b + c * d
+__device__ __forceinline__ CDD cdot(double2 a, const CDD& b, double2 c, const CDD& d) {
+  const DD z{0.0, 0.0};
+  return CDD{dd_fma(-c.y, d.y, dd_fma(c.x, d.x, dd_fma(-a.y, b.y, dd_fma(a.x, b.x, z)))),
+             dd_fma(c.y, d.x, dd_fma(c.x, d.y, dd_fma(a.y, b.x, dd_fma(a.x, b.y, z))))};
+}
+
 }  // namespace mb

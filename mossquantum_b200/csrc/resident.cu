@@ -29,6 +29,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "fusemat.cuh"
 #include "internal.h"
 
 namespace mb {
@@ -150,31 +151,6 @@ __device__ __forceinline__ void apply(const M2& m, double2& x, double2& y) {
   const double2 a = x, b = y;
   x = cfma(m.m01, b, cmul(m.m00, a));
   y = cfma(m.m11, b, cmul(m.m10, a));
-}
-
-// A run's product is rounded once: its entries are carried as high and low parts, because an error
-// of the matrix is the same for every amplitude and adds up over the steps, where roundings of
-// amplitudes average out.
-struct DD {
-  double h, l;
-};
-__device__ __forceinline__ DD dd_fma(double a, DD b, DD c) {
-  const double p = a * b.h, q = fma(a, b.h, -p) + a * b.l;     // a * b
-  const double s = c.h + p, z = s - c.h;
-  const double r = ((c.h - (s - z)) + (p - z)) + (c.l + q);    // two-sum of the high parts
-  const double h = s + r;
-  return DD{h, r - (h - s)};
-}
-struct CDD {
-  DD x, y;
-};
-__device__ __forceinline__ CDD wide(double2 a) { return CDD{DD{a.x, 0.0}, DD{a.y, 0.0}}; }
-__device__ __forceinline__ double2 narrow(const CDD& a) { return make_double2(a.x.h, a.y.h); }
-// a * b + c * d
-__device__ __forceinline__ CDD cdot(double2 a, const CDD& b, double2 c, const CDD& d) {
-  const DD z{0.0, 0.0};
-  return CDD{dd_fma(-c.y, d.y, dd_fma(c.x, d.x, dd_fma(-a.y, b.y, dd_fma(a.x, b.x, z)))),
-             dd_fma(c.y, d.x, dd_fma(c.x, d.y, dd_fma(a.y, b.x, dd_fma(a.x, b.y, z))))};
 }
 
 // Storage index of pair q: a zero inserted at the pivot.
