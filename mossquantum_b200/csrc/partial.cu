@@ -78,13 +78,17 @@ __global__ void __launch_bounds__(256) k_partial_trace_dm(const double2* __restr
 // accumulate BS x BS micro-tiles (rows a, a + nb, ...: consecutive threads read consecutive
 // shared words). r is Hermitian: only block pairs ia <= ic and, on the diagonal pair, only
 // micro-tiles i <= j are formed; spare threads take further columns (`groups`). Chunks of t keep
-// every SM busy (one CTA of nine warps each: the accumulators give every thread 64 independent
+// every SM busy (one CTA each: the accumulators give every thread 64 independent
 // FP64 chains, and a second CTA would make them spill); k_partial_sum adds the chunks in order
 // and writes both halves of r.
-// 22 qubits, 6 kept: 93 us and 6 us for the sum, against 34.5 ms with one thread per entry of r
+// 22 qubits, 6 kept: 85 us and 6 us for the sum, against 34.5 ms with one thread per entry of r
 // looping over t; the floor is 31 us of FP64 (2^28 complex multiply-adds, half of them by symmetry).
 constexpr int kPTBits = 11;        // log2 of a staged tile's amplitudes
-constexpr int kPTThreads = 288;    // 256 micro-tiles of a block pair, or twice 136 of a diagonal one
+// Threads: 256 micro-tiles of a block pair, or three times 136 of the one block there is up to six
+// kept qubits (twice 136 leave nine warps on four schedulers: 93 us, thirteen 85; at 22 qubits, 6 kept). Pairs have the
+// registers to run two columns at once (22 qubits, 8 kept: the call 558 -> 520 us); with 416 threads
+// two measured the same as one.
+constexpr int kPTThreads = 288, kPTThreadsOne = 416;
 
 struct TraceArgs {
   int n, m, k, ma, tb;             // qubits, kept, traced; row and column bits of a tile
@@ -118,8 +122,8 @@ __device__ __forceinline__ void put_entry(double2* out, const TraceArgs& a, int 
   if (ia != ic || i != j) out[col + (row << a.m)] = cconj(v);
 }
 
-template <int BS>
-__global__ void __launch_bounds__(kPTThreads, 1) k_partial_outer(const double2* __restrict__ in, const TraceArgs a,
+template <int BS, int NT>
+__global__ void __launch_bounds__(NT, 1) k_partial_outer(const double2* __restrict__ in, const TraceArgs a,
                                                                 double2* __restrict__ part,
                                                                 double2* __restrict__ out) {
   extern __shared__ double2 sm[];
@@ -134,7 +138,7 @@ __global__ void __launch_bounds__(kPTThreads, 1) k_partial_outer(const double2* 
   uint16_t* slot = reinterpret_cast<uint16_t*>(goff + E);
   // Staging map: element e's bits, in ascending address order, are the tile's ma kept and tb
   // traced bits (the lowest of each kind).
-  for (int e = threadIdx.x; e < E; e += kPTThreads) {
+  for (int e = threadIdx.x; e < E; e += NT) {
     uint64_t off = 0;
     int row = 0, col = 0;
     for (int x = 0, y = 0, j = 0; x < a.ma || y < a.tb; ++j) {
@@ -161,7 +165,7 @@ __global__ void __launch_bounds__(kPTThreads, 1) k_partial_outer(const double2* 
   auto stage = [&](int64_t s, int which) {
     const int64_t t = base_t(s);
     double2* d = buf + size_t(which) * nbuf * E;
-    for (int e = threadIdx.x; e < E; e += kPTThreads) {
+    for (int e = threadIdx.x; e < E; e += NT) {
       cp16(d + slot[e], src + (hi_a | t | goff[e]));
       if (!diag) cp16(d + E + slot[e], src + (hi_c | t | goff[e]));
     }
@@ -169,7 +173,7 @@ __global__ void __launch_bounds__(kPTThreads, 1) k_partial_outer(const double2* 
   };
   const int nb = A / BS;                            // micro-tile rows
   const int P = diag ? nb * (nb + 1) / 2 : nb * nb; // micro-tiles
-  const int groups = kPTThreads / P;
+  const int groups = NT / P;
   const int g = threadIdx.x / P, p = threadIdx.x - g * P;
   const bool on = g < groups;
   int i = 0, j = 0;
@@ -197,7 +201,7 @@ __global__ void __launch_bounds__(kPTThreads, 1) k_partial_outer(const double2* 
     const double2* ra = buf + size_t(s & 1) * nbuf * E;
     const double2* rc = diag ? ra : ra + E;
     if (on) {
-#pragma unroll 1
+#pragma unroll NT == kPTThreads ? 2 : 1
       for (int t = g; t < T; t += groups) {
         double2 x[BS];
 #pragma unroll
@@ -221,14 +225,14 @@ __global__ void __launch_bounds__(kPTThreads, 1) k_partial_outer(const double2* 
     if (groups > 1) {
 #pragma unroll
       for (int c = 0; c < BS; ++c)
-        if (on) red[c * kPTThreads + threadIdx.x] = acc[r][c];
+        if (on) red[c * NT + threadIdx.x] = acc[r][c];
       __syncthreads();
       for (int n = groups; n > 1;) {
         const int half = (n + 1) / 2;
         if (g < n - half)
 #pragma unroll
           for (int c = 0; c < BS; ++c) {
-            double2* x = red + c * kPTThreads + threadIdx.x;
+            double2* x = red + c * NT + threadIdx.x;
             *x = cadd(*x, x[half * P]);
           }
         __syncthreads();
@@ -236,7 +240,7 @@ __global__ void __launch_bounds__(kPTThreads, 1) k_partial_outer(const double2* 
       }
       if (g == 0)
 #pragma unroll
-        for (int c = 0; c < BS; ++c) acc[r][c] = red[c * kPTThreads + threadIdx.x];
+        for (int c = 0; c < BS; ++c) acc[r][c] = red[c * NT + threadIdx.x];
       __syncthreads();
     }
     if (on && g == 0)
@@ -356,19 +360,21 @@ int trace_pure_bs(mb_state in, TraceArgs a, mb_state out) {
   // one staged tile; shorter chunks spend their time on the pipeline's start and on partial tiles).
   a.chunks = int(std::max<int64_t>(1, std::min<int64_t>(steps / 4, g_ctx.sm_count / (int64_t(a.npairs) * B))));
   const size_t E = size_t(1) << (a.ma + a.tb);
+  const int nt = a.nblocks > 1 ? kPTThreads : kPTThreadsOne;
+  auto* outer = a.nblocks > 1 ? k_partial_outer<BS, kPTThreads> : k_partial_outer<BS, kPTThreadsOne>;
   const size_t shm = std::max(E * ((a.nblocks > 1 ? 4 : 2) * sizeof(double2) + sizeof(uint32_t) + sizeof(uint16_t)),
-                              sizeof(double2) * size_t(BS * kPTThreads));
+                              sizeof(double2) * size_t(BS * nt));
   const int64_t per = int64_t(a.npairs) * a.chunks * a.entries;
   double2* part = nullptr;
   if (a.chunks > 1 && dev_alloc((void**)&part, sizeof(double2) * size_t(per) * B)) a.chunks = 1;  // no room: unsplit
-  cudaFuncSetAttribute(k_partial_outer<BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm));
+  cudaFuncSetAttribute(outer, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shm));
   int rc = MB_OK;
   for (int b0 = 0; b0 < B && !rc; b0 += 65535) {    // grid.z limit
     const int nbat = std::min(65535, B - b0);
     const double2* src = in->d + (int64_t(b0) << a.n);
     double2* dst = out->d + (int64_t(b0) << (2 * a.m));
     double2* pt = part ? part + per * b0 : nullptr;
-    k_partial_outer<BS><<<dim3(a.npairs, a.chunks, nbat), kPTThreads, shm, g_ctx.stream>>>(src, a, pt, dst);
+    outer<<<dim3(a.npairs, a.chunks, nbat), nt, shm, g_ctx.stream>>>(src, a, pt, dst);
     ++launch_counter();
     if (a.chunks > 1) {
       const int64_t work = int64_t(nbat) * a.npairs * a.entries, cap = int64_t(g_ctx.sm_count) * 32;
