@@ -478,6 +478,8 @@ struct Schedule {
   FuseComp* d_fcomps = nullptr;
   FuseRec* d_frecs = nullptr;
   int N = 0, dm = 0, t = 0, R = 0, nsamples = 1;
+  int asked = 0;        // register width looked up (R, or 4 where a schedule of width 3 took its place)
+  bool strict = false;  // specialised kernels for every pass, or none
   int lo = 0, hi = -1;  // instruction range [lo, hi) of the circuit
   int adjoint = 0;      // reverse sweep with gradient accumulators
   int* d_gslots = nullptr;
@@ -1995,6 +1997,7 @@ static int plain_fop_launch(mb_circuit c, const FOp& f, double2* v, int64_t elem
 struct Tuning {
   int t = 12, R = 4;
   int fuse = 1;   // fusion width: 1 = single-qubit runs fused at bind time, 0 = one micro-op per gate
+  bool rule = false;  // R = 4 by the rule below: rebuilt with 3 unless every pass is specialised
 };
 
 std::mutex g_tune_mu;
@@ -2034,7 +2037,9 @@ static Tuning tuning_for(int N, bool whole = true) {
     // gradient are mostly light passes (24 qubits: 6.50 against 6.36 ms). 32 amplitudes with
     // 6 warps: no faster, compile times past the budget. 2^11 tiles: 5.62 against 5.43 ms (25 qubits).
     tu.t = 10;
-    tu.R = N >= 20 && whole ? 4 : 3;
+    // Sources grow with R, so a schedule with a pass beyond the source limit takes R = 3.
+    tu.rule = N >= 20 && whole;
+    tu.R = tu.rule ? 4 : 3;
   }
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -2042,12 +2047,16 @@ static Tuning tuning_for(int N, bool whole = true) {
     if (it != g_tuning.end()) {
       tu.t = it->second.first;
       tu.R = it->second.second;
+      tu.rule = false;
     }
     auto fi = g_fusion.find(N);
     if (fi != g_fusion.end()) tu.fuse = fi->second;
   }
   if (const char* e = getenv("MB_TILE_BITS")) tu.t = std::max(8, std::min(12, atoi(e)));
-  if (const char* e = getenv("MB_REG_BITS")) tu.R = std::max(3, std::min(5, atoi(e)));
+  if (const char* e = getenv("MB_REG_BITS")) {
+    tu.R = std::max(3, std::min(5, atoi(e)));
+    tu.rule = false;
+  }
   tu.t = std::min(tu.t, N);
   return tu;
 }
@@ -2070,6 +2079,7 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
   if (force) {
     tu.t = std::min(force->t, N);
     tu.R = force->R;
+    tu.rule = false;
   }
   if (adjoint) {
     // y and delta tiles, double-buffered: MB_ADJOINT_TILE_BITS (8..11) and the register width of
@@ -2095,7 +2105,7 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
     return s->nsamples > 1 && s->nsamples >= nsamples;
   };
   for (Schedule* s : c->scheds)
-    if (s->N == N && s->dm == dm && !s->dagger && s->t == tu.t && s->R == tu.R && fits(s) &&
+    if (s->N == N && s->dm == dm && !s->dagger && s->t == tu.t && s->asked == tu.R && fits(s) &&
         (adjoint || s->fuse == (tu.fuse != 0)) &&
         s->lo == lo && s->hi == hi && s->adjoint == adjoint && s->tile_only == tile_only) {
       *out = s;
@@ -2110,7 +2120,7 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
   S->N = N;
   S->dm = dm;
   S->t = tu.t;
-  S->R = tu.R;
+  S->R = S->asked = tu.R;
   S->nsamples = nsamples;
   S->lo = lo;
   S->hi = hi;
@@ -2202,6 +2212,26 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
                                     cudaMemcpyHostToDevice, g_ctx.stream));
   }
   MB_CHECK_CUDA(cudaStreamSynchronize(g_ctx.stream));
+  auto drop = [&] {
+    dev_free(S->d_stages);
+    dev_free(S->d_mops);
+    dev_free(S->d_gslots);
+    dev_free(S->d_xtab);
+    dev_free(S->d_frecs);
+    dev_free(S->d_fcomps);
+  };
+  if (!adjoint && !tile_only && tu.rule) {
+    S->strict = true;
+    prepare_jit(S.get());
+    if (S->jit != 1) {
+      drop();
+      Tuning three = tu;
+      three.R = 3;
+      const int rc3 = get_schedule_impl(c, n, dm, adjoint, lo, hi, nsamples, &three, tile_only, out);
+      if (rc3 == MB_OK && (*out)->R == 3) (*out)->asked = 4;
+      return rc3;
+    }
+  }
   if (!adjoint && !tile_only && S->R == 3 && !getenv("MB_REG_BITS")) {
     // Register width 3 exists only as specialised kernels: if they cannot all be built (source
     // limits, compile budget), use width 4 for this register size from now on. (A width forced
@@ -2214,13 +2244,8 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_tuning[N] = {S->t, 4};
       }
-      dev_free(S->d_stages);
-      dev_free(S->d_mops);
-      dev_free(S->d_gslots);
-      dev_free(S->d_xtab);
-      dev_free(S->d_frecs);
-      dev_free(S->d_fcomps);
-      return get_schedule_impl(c, n, dm, adjoint, lo, hi, nsamples, force, tile_only, out);
+      drop();
+      return get_schedule_impl(c, n, dm, adjoint, lo, hi, nsamples, nullptr, tile_only, out);
     }
   }
   *out = S.get();
@@ -2359,7 +2384,7 @@ static void prepare_jit(Schedule* S) {
   if (const char* e = getenv("MB_JIT_BUDGET_S")) budget = atof(e);
   size_t max_src = size_t(128) << 10;
   if (const char* e = getenv("MB_JIT_MAX_SOURCE_KB")) max_src = size_t(std::max(1, atoi(e))) << 10;
-  const bool partial_ok = !S->adjoint && (S->R == 4 || S->R == 5);
+  const bool partial_ok = !S->adjoint && (S->R == 4 || S->R == 5) && !S->strict;
   if (S->adjoint) max_src *= 4;  // no interpreter to fall back on: only refuse the extreme ones
   std::vector<std::string> small;
   std::vector<Pass*> small_who;
