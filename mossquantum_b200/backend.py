@@ -53,7 +53,7 @@ def supports(b, operation, state, action="apply") -> bool:
         return False
     if action == "expectation":
         if isinstance(operation, (QubitsTerm, QubitsOperator)):
-            return as_operator(operation).reach()[1] <= 5
+            return all(len(t.positions) <= 5 for t in as_operator(operation).terms)
         return False
     if action == "probabilities":
         return True
@@ -152,7 +152,7 @@ def expectation(observable, state):
     if not supports(_BACKEND, observable, state, "expectation"):
         raise UnsupportedOperation(f"B200Backend cannot take the expectation of {type(observable).__name__}")
     op = as_operator(observable)
-    if op.reach()[0] > state.n:
+    if op.nqubits() > state.n:
         raise ValueError("observable acts outside the register")
     out = np.zeros(2 * max(state.batch, 1))
     if state.batch == 0:

@@ -73,7 +73,7 @@ class ExpectationObjective:
             compiled = known[0]
         if not supports(backend(state), op, state, "expectation"):
             raise N.UnsupportedOperation("B200Backend cannot take the expectation of this observable")
-        if op.reach()[0] > state.n:
+        if op.nqubits() > state.n:
             raise ValueError("observable acts outside the register")
         theta = compiled.theta_from(slots)
         out = np.zeros(2 * state.batch)

@@ -127,7 +127,7 @@ class QubitsOperator:
         return len(self.terms)
 
     def nqubits(self):
-        return max((t.nqubits() for t in self.terms), default=0)
+        return max(itertools.chain.from_iterable([t.positions for t in self.terms]), default=0)
 
     def specs(self):
         return [t.spec() for t in self.terms]
@@ -154,11 +154,6 @@ class QubitsOperator:
                     b"".join(itertools.chain.from_iterable([t.op for t in terms])))
         except (BufferError, TypeError, ValueError):
             return None
-
-    def reach(self):
-        """(highest site, most sites of a term)."""
-        at = [t.positions for t in self.terms]
-        return max((max(p) for p in at if p), default=0), max(map(len, at), default=0)
 
     def is_hermitian(self):
         """Kept under the terms' values."""
