@@ -65,12 +65,12 @@ def test_unknown_types_are_not_remembered():
 
 def test_operator_checks_follow_the_terms():
     op = mq.QubitsOperator([mq.QubitsTerm([1, 3], ["X", "Z"], 0.5), mq.QubitsTerm([2], ["Y"], -1.0)])
-    assert op.reach() == (3, 2) and op.is_hermitian()
+    assert op.nqubits() == 3 and op.is_hermitian()
     op.terms[1].op[0][0, 1] = 3.0
     assert not op.is_hermitian()
     op.terms[1].op[0][0, 1] = -1j
     assert op.is_hermitian()
     op.add(mq.QubitsTerm([1, 2, 4], ["Z"] * 3, 1j))
-    assert op.reach() == (4, 3) and not op.is_hermitian()
+    assert op.nqubits() == 4 and not op.is_hermitian()
     pair = mq.QubitsOperator([mq.QubitsTerm([1], ["+"], 1.0), mq.QubitsTerm([1], ["-"], 1.0)])
     assert pair.is_hermitian() and mq.QubitsOperator([]).is_hermitian()
