@@ -26,6 +26,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <string>
 #include <unordered_map>
 
@@ -178,7 +179,7 @@ __device__ __forceinline__ CDD lane_of(const CDD& v, int src) {
 // entry (r, c); every component is read by the lanes that hold its entries (a 2x2 inside a 4x4
 // widened by zeros) and multiplied through shuffles. Bound by the latency of a component's two
 // dependent reads (offset, entry), so four components are read together: 40 records of up to 16
-// components (density matrix of 10 qubits) took 45 us with one thread per record, now 19. All lanes of
+// components (density matrix of 10 qubits) took 45 us with one thread per record, now 21. All lanes of
 // the warp enter (a lane without a record passes nc = 0): groups run to the longest record of the warp.
 // 2x2 products are kept in double-double and rounded once: a product's error acts alike on every
 // amplitude of a state (gradients of 20 and 22 qubits, 16 sets of angles, largest error relative to the
@@ -1997,11 +1998,12 @@ static int plain_fop_launch(mb_circuit c, const FOp& f, double2* v, int64_t elem
 struct Tuning {
   int t = 12, R = 4;
   int fuse = 1;   // fusion width: 1 = single-qubit runs fused at bind time, 0 = one micro-op per gate
-  bool rule = false;  // R = 4 by the rule below: rebuilt with 3 unless every pass is specialised
+  bool strict = false;  // rebuilt with R = 3 unless every pass is specialised
 };
 
 std::mutex g_tune_mu;
 std::map<int, std::pair<int, int>> g_tuning;  // register bits -> (tile bits, register bits)
+std::set<int> g_partial;                       // register bits whose width 4 may run partly interpreted
 std::map<int, int> g_fusion;                   // register bits -> fusion width
 
 // Specialised kernels are used from MB_JIT_MIN_BITS register bits on (default 18); MB_JIT=0
@@ -2037,9 +2039,9 @@ static Tuning tuning_for(int N, bool whole = true) {
     // gradient are mostly light passes (24 qubits: 6.50 against 6.36 ms). 32 amplitudes with
     // 6 warps: no faster, compile times past the budget. 2^11 tiles: 5.62 against 5.43 ms (25 qubits).
     tu.t = 10;
-    // Sources grow with R, so a schedule with a pass beyond the source limit takes R = 3.
-    tu.rule = N >= 20 && whole;
-    tu.R = tu.rule ? 4 : 3;
+    // Sources grow with R, so a schedule with a pass beyond the source limit takes R = 3 (unless that
+    // failed as well), however its R = 4 was chosen.
+    tu.R = N >= 20 && whole ? 4 : 3;
   }
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -2047,15 +2049,15 @@ static Tuning tuning_for(int N, bool whole = true) {
     if (it != g_tuning.end()) {
       tu.t = it->second.first;
       tu.R = it->second.second;
-      tu.rule = false;
     }
     auto fi = g_fusion.find(N);
     if (fi != g_fusion.end()) tu.fuse = fi->second;
+    tu.strict = tu.t == 10 && tu.R == 4 && N >= 20 && !g_partial.count(N) && want_jit(N) && jit_available();
   }
   if (const char* e = getenv("MB_TILE_BITS")) tu.t = std::max(8, std::min(12, atoi(e)));
   if (const char* e = getenv("MB_REG_BITS")) {
     tu.R = std::max(3, std::min(5, atoi(e)));
-    tu.rule = false;
+    tu.strict = false;
   }
   tu.t = std::min(tu.t, N);
   return tu;
@@ -2079,7 +2081,7 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
   if (force) {
     tu.t = std::min(force->t, N);
     tu.R = force->R;
-    tu.rule = false;
+    tu.strict = false;
   }
   if (adjoint) {
     // y and delta tiles, double-buffered: MB_ADJOINT_TILE_BITS (8..11) and the register width of
@@ -2220,7 +2222,7 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
     dev_free(S->d_frecs);
     dev_free(S->d_fcomps);
   };
-  if (!adjoint && !tile_only && tu.rule) {
+  if (!adjoint && !tile_only && tu.strict) {
     S->strict = true;
     prepare_jit(S.get());
     if (S->jit != 1) {
@@ -2243,6 +2245,7 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
       {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_tuning[N] = {S->t, 4};
+        g_partial.insert(N);
       }
       drop();
       return get_schedule_impl(c, n, dm, adjoint, lo, hi, nsamples, nullptr, tile_only, out);
