@@ -231,7 +231,7 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
     // small pure states: values and gradient in one launch
     bool done = false;
     std::vector<double2> v(B);
-    if ((rc = resident_run(c, o, init, theta, w.data(), v.data(), grad, &done))) return rc;
+    if ((rc = resident_run(c, o, init, theta, w.data(), checkpoint_every, v.data(), grad, &done))) return rc;
     if (done) {
       double total = 0;
       for (int b = 0; b < B; ++b) total += w[b] * v[b].x;

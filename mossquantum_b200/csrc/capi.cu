@@ -1128,7 +1128,7 @@ extern "C" int mb_objective_values(mb_circuit c, mb_observable o, mb_state init,
     return MB_EUNSUPPORTED;
   }
   bool done = false;
-  if (int rc = resident_run(c, o, init, theta, nullptr, reinterpret_cast<double2*>(out), nullptr, &done)) return rc;
+  if (int rc = resident_run(c, o, init, theta, nullptr, 0, reinterpret_cast<double2*>(out), nullptr, &done)) return rc;
   if (done) return MB_OK;
   // The general form: a private copy of the initial state through the fused passes.
   const bool init_dm = init->kind == MB_DENSITY || init->kind == MB_BATCH_DENSITY;

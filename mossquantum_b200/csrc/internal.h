@@ -183,9 +183,10 @@ int reverse_dm_single(mb_circuit c, int n, const double2* ckpt, double2* delta, 
 
 // resident.cu: small pure states, the whole objective in one launch. values: <H> per sample;
 // grad (or null): the gradient of the weighted sum. *done = false when the circuit, the
-// observable or the size has no resident form (nothing has been launched then).
+// observable or the size has no resident form, or checkpoints (checkpoint_every > 0) would change
+// the gradient (nothing has been launched then).
 int resident_run(mb_circuit c, mb_observable o, mb_state init, const double* theta, const double* weights,
-                 double2* values, double* grad, bool* done);
+                 int checkpoint_every, double2* values, double* grad, bool* done);
 void resident_release(mb_circuit c);
 
 // pauli.cu
