@@ -776,26 +776,24 @@ int theta_stage(mb_circuit c, const double* theta, size_t ntheta, int rows) {
     if ((rc = dev_alloc((void**)&c->d_theta, sizeof(double) * need))) return rc;
     c->theta_cap = need;
   }
-  if (ntheta) {
-    if (ntheta > kThetaStage) {
-      // pageable source: the copy has left it when the call returns
-      MB_CHECK_CUDA(cudaMemcpyAsync(c->d_theta, theta, sizeof(double) * ntheta, cudaMemcpyHostToDevice, g_ctx.stream));
-      return MB_OK;
-    }
+  // The caller's memory may be page-locked, and a copy from it would still be reading after the return, so
+  // every value goes through a buffer of the ring; long lists take several.
+  for (size_t at = 0; at < ntheta; at += kThetaStage) {
+    const size_t count = std::min(ntheta - at, kThetaStage);
     auto& h = g_ctx.h_theta[g_ctx.h_theta_next];
     g_ctx.h_theta_next = (g_ctx.h_theta_next + 1) % 8;
     if (!h.copied) MB_CHECK_CUDA(cudaEventCreateWithFlags(&h.copied, cudaEventDisableTiming));
     else MB_CHECK_CUDA(cudaEventSynchronize(h.copied));
-    if (h.cap < ntheta) {
-      const size_t cap = std::max<size_t>(4096, 2 * ntheta);
+    if (h.cap < count) {
+      const size_t cap = std::min(kThetaStage, std::max<size_t>(4096, 2 * count));
       if (h.p) cudaFreeHost(h.p);
       h.p = nullptr;
       h.cap = 0;
       MB_CHECK_CUDA(cudaMallocHost((void**)&h.p, sizeof(double) * cap));
       h.cap = cap;
     }
-    std::memcpy(h.p, theta, sizeof(double) * ntheta);
-    MB_CHECK_CUDA(cudaMemcpyAsync(c->d_theta, h.p, sizeof(double) * ntheta, cudaMemcpyHostToDevice, g_ctx.stream));
+    std::memcpy(h.p, theta + at, sizeof(double) * count);
+    MB_CHECK_CUDA(cudaMemcpyAsync(c->d_theta + at, h.p, sizeof(double) * count, cudaMemcpyHostToDevice, g_ctx.stream));
     MB_CHECK_CUDA(cudaEventRecord(h.copied, g_ctx.stream));
   }
   return MB_OK;

@@ -111,9 +111,9 @@ struct Ctx {
   double* h_small = nullptr;        // small synchronous calls: pinned staging and its device side
   double* d_small = nullptr;
   size_t h_small_cap = 0, d_small_cap = 0;
-  // Pinned staging for theta uploads of at most kThetaStage doubles, used in turn: a buffer is
-  // reused once its own copy has been made, so callers run ahead of the device instead of
-  // waiting for it. Larger uploads go from the caller's memory. Freed by mb_shutdown.
+  // Pinned staging for theta uploads, kThetaStage doubles at most in each buffer, used in turn: a
+  // buffer is reused once its own copy has been made, so callers run ahead of the device instead of
+  // waiting for it. Freed by mb_shutdown.
   struct ThetaBuf {
     double* p = nullptr;
     size_t cap = 0;
