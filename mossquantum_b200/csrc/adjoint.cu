@@ -191,6 +191,8 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
                           const double* weights, int checkpoint_every, double* value, double* grad) {
   std::lock_guard<std::recursive_mutex> lk(g_mu);
   if (int rc = check_init()) return rc;
+  // (an upload recorded into a graph would also leave its staging buffer's event unusable)
+  if (int rc = check_not_capturing("mb_adjoint")) return rc;
   if (!c || !o || !init || !value || (!grad && c->nslots) || (!theta && ntheta)) return MB_EINVAL;
   if (init->n != c->n) {
     set_error("circuit compiled for %d qubits, initial state has %d", c->n, init->n);
