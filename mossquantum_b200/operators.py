@@ -163,9 +163,9 @@ class QubitsOperator:
         return self._hermitian[1]
 
     def _check_hermitian(self):
-        if all(np.imag(t.coeff) == 0 for t in self.terms):
+        if all(np.imag(t.coeff) == 0 and np.isfinite(t.coeff) for t in self.terms):
             m = np.array([o for t in self.terms for o in t.op]).reshape(-1, 2, 2)
-            if np.array_equal(m, m.conj().transpose(0, 2, 1)):
+            if np.array_equal(m, m.conj().transpose(0, 2, 1)) and np.isfinite(m).all():
                 return True      # real combinations of products of Hermitian matrices
         keys = {}
         for t in self.terms:
