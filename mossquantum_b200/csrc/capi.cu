@@ -1078,6 +1078,18 @@ int expect_keys(mb_observable o, mb_state s, double2* out) {
   return MB_OK;
 }
 
+// MB_EXPECT_KEYS=1 keeps every expectation on the dense keys.
+bool expect_keys_only() {
+  const char* e = getenv("MB_EXPECT_KEYS");
+  return e && atoi(e) != 0;
+}
+
+// <H> per sample into g_ctx.results: Pauli passes on pure states, else key by key.
+static int expect_state(mb_observable o, mb_state s) {
+  const int is_dm = s->kind == MB_DENSITY || s->kind == MB_BATCH_DENSITY;
+  return !is_dm && o->pauli_ok && !expect_keys_only() ? expect_pauli(o, s) : expect_keys(o, s);
+}
+
 int validate_observable(mb_observable o, mb_state s) {
   if (o->max_site >= s->n && !o->keys.empty() && !(o->keys.size() == 1 && o->keys[0].k == 0)) {
     set_error("observable acts on qubit %d of a %d-qubit state", o->max_site + 1, s->n);
@@ -1099,9 +1111,7 @@ extern "C" int mb_expect(mb_observable o, mb_state s, double* out) {
     set_error("at most 65536 samples per expectation call");
     return MB_EUNSUPPORTED;
   }
-  const int is_dm = s->kind == MB_DENSITY || s->kind == MB_BATCH_DENSITY;
-  const bool keys_only = getenv("MB_EXPECT_KEYS") && atoi(getenv("MB_EXPECT_KEYS")) != 0;
-  int rc = (!is_dm && o->pauli_ok && !keys_only) ? expect_pauli(o, s) : expect_keys(o, s);
+  int rc = expect_state(o, s);
   if (rc) return rc;
   MB_CHECK_CUDA(cudaMemcpyAsync(out, g_ctx.results, sizeof(double2) * s->batch, cudaMemcpyDeviceToHost, g_ctx.stream));
   MB_CHECK_CUDA(cudaStreamSynchronize(g_ctx.stream));
@@ -1125,9 +1135,11 @@ extern "C" int mb_objective_values(mb_circuit c, mb_observable o, mb_state init,
     set_error("at most 65536 samples per expectation call");
     return MB_EUNSUPPORTED;
   }
-  bool done = false;
-  if (int rc = resident_run(c, o, init, theta, nullptr, 0, reinterpret_cast<double2*>(out), nullptr, &done)) return rc;
-  if (done) return MB_OK;
+  if (!expect_keys_only()) {
+    bool done = false;
+    if (int rc = resident_run(c, o, init, theta, nullptr, 0, reinterpret_cast<double2*>(out), nullptr, &done)) return rc;
+    if (done) return MB_OK;
+  }
   // The general form: a private copy of the initial state through the fused passes.
   const bool init_dm = init->kind == MB_DENSITY || init->kind == MB_BATCH_DENSITY;
   const int kind = init_dm || !c->has_channel ? init->kind : init->kind == MB_PURE ? MB_DENSITY : MB_BATCH_DENSITY;
@@ -1141,7 +1153,7 @@ extern "C" int mb_objective_values(mb_circuit c, mb_observable o, mb_state init,
   }
   if (!rc) rc = bind_circuit(c, theta, ntheta, 1);
   if (!rc) rc = apply_fused(c, s, 0);
-  if (!rc) rc = (o->pauli_ok && !init_dm && kind == init->kind) ? expect_pauli(o, s) : expect_keys(o, s);
+  if (!rc) rc = expect_state(o, s);
   if (!rc) {
     cudaMemcpyAsync(out, g_ctx.results, sizeof(double2) * s->batch, cudaMemcpyDeviceToHost, g_ctx.stream);
     const cudaError_t e = cudaStreamSynchronize(g_ctx.stream);

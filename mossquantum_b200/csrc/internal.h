@@ -158,6 +158,7 @@ int apply_plain(mb_circuit c, mb_state s, int64_t mrow_stride);
 int validate_apply(mb_circuit c, mb_state s);
 int validate_observable(mb_observable o, mb_state s);
 int expect_keys(mb_observable o, mb_state s, double2* out = nullptr);
+bool expect_keys_only();
 int observable_apply(mb_observable o, const double2* in, double2* out, int n, int is_dm, int nsamples);
 
 // fused.cu

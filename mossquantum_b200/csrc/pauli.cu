@@ -460,8 +460,7 @@ bool observable_strings(mb_observable o, int n, ObsStrings* out) {
 // key); products of general 2x2 matrices on many sites, with up to 4^k strings, stay on the
 // dense keys (MB_EXPECT_KEYS=1 keeps every observable there).
 static bool dm_strings(mb_observable o, int n) {
-  const char* keys = getenv("MB_EXPECT_KEYS");
-  if (keys && atoi(keys) != 0) return false;
+  if (expect_keys_only()) return false;
   const PauliData* pd = o->pauli;
   ObsStrings os;
   return observable_strings(o, n, &os) && os.nstr > 0 && int64_t(os.nstr) <= 4 * pd->dense_rows;
