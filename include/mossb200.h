@@ -225,7 +225,8 @@ MB_API int mb_uneven_apply(mb_uneven u, int flags);
 MB_API int mb_uneven_info(mb_uneven u, int* persistent_groups, int* fallback_groups, int* samples);
 MB_API int mb_uneven_free(mb_uneven u);
 
-/* ---- tuning: tile bits t (10..12) and register bits R (3..5) per register size ---------- */
+/* ---- tuning: tile bits t (10..12) and register bits R (3..5) per register size ----------
+ * What a schedule of the size is built with; one whose kernels are too long for it falls back by itself. */
 MB_API int mb_tuning_set(int nbits, int tile_bits, int reg_bits);
 MB_API int mb_tuning_get(int nbits, int* tile_bits, int* reg_bits);
 /* Fusion width per register size: 1 (default) multiplies every run of operations on one qubit

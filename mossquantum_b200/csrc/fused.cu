@@ -26,7 +26,6 @@
 #include <map>
 #include <memory>
 #include <mutex>
-#include <set>
 #include <string>
 #include <unordered_map>
 
@@ -479,7 +478,7 @@ struct Schedule {
   FuseComp* d_fcomps = nullptr;
   FuseRec* d_frecs = nullptr;
   int N = 0, dm = 0, t = 0, R = 0, nsamples = 1;
-  int asked = 0;        // register width looked up (R, or 4 where a schedule of width 3 took its place)
+  int asked = 0;        // register width it was looked up with; R differs where it fell back
   bool strict = false;  // specialised kernels for every pass, or none
   int lo = 0, hi = -1;  // instruction range [lo, hi) of the circuit
   int adjoint = 0;      // reverse sweep with gradient accumulators
@@ -1998,12 +1997,12 @@ static int plain_fop_launch(mb_circuit c, const FOp& f, double2* v, int64_t elem
 struct Tuning {
   int t = 12, R = 4;
   int fuse = 1;   // fusion width: 1 = single-qubit runs fused at bind time, 0 = one micro-op per gate
-  bool strict = false;  // rebuilt with R = 3 unless every pass is specialised
+  bool strict = false;  // R = 4 only if every pass is specialised, else R = 3
+  int asked = 0;        // width that a fallback stands for (0: R itself)
 };
 
 std::mutex g_tune_mu;
 std::map<int, std::pair<int, int>> g_tuning;  // register bits -> (tile bits, register bits)
-std::set<int> g_partial;                       // register bits whose width 4 may run partly interpreted
 std::map<int, int> g_fusion;                   // register bits -> fusion width
 
 // Specialised kernels are used from MB_JIT_MIN_BITS register bits on (default 18); MB_JIT=0
@@ -2039,8 +2038,8 @@ static Tuning tuning_for(int N, bool whole = true) {
     // gradient are mostly light passes (24 qubits: 6.50 against 6.36 ms). 32 amplitudes with
     // 6 warps: no faster, compile times past the budget. 2^11 tiles: 5.62 against 5.43 ms (25 qubits).
     tu.t = 10;
-    // Sources grow with R, so a schedule with a pass beyond the source limit takes R = 3 (unless that
-    // failed as well), however its R = 4 was chosen.
+    // Sources grow with R, so a schedule with a pass beyond the source limit takes R = 3, however its
+    // R = 4 was chosen, and R = 4 partly interpreted where that fails as well.
     tu.R = N >= 20 && whole ? 4 : 3;
   }
   {
@@ -2052,7 +2051,7 @@ static Tuning tuning_for(int N, bool whole = true) {
     }
     auto fi = g_fusion.find(N);
     if (fi != g_fusion.end()) tu.fuse = fi->second;
-    tu.strict = tu.t == 10 && tu.R == 4 && N >= 20 && !g_partial.count(N) && want_jit(N) && jit_available();
+    tu.strict = tu.t == 10 && tu.R == 4 && N >= 20 && want_jit(N) && jit_available();
   }
   if (const char* e = getenv("MB_TILE_BITS")) tu.t = std::max(8, std::min(12, atoi(e)));
   if (const char* e = getenv("MB_REG_BITS")) {
@@ -2082,6 +2081,7 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
     tu.t = std::min(force->t, N);
     tu.R = force->R;
     tu.strict = false;
+    tu.asked = force->asked;
   }
   if (adjoint) {
     // y and delta tiles, double-buffered: MB_ADJOINT_TILE_BITS (8..11) and the register width of
@@ -2102,12 +2102,13 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
   if (!adjoint && nsamples > 1)
     for (cap = 2; cap < nsamples; cap *= 2) {
     }
+  const int asked = tu.asked ? tu.asked : tu.R;
   auto fits = [&](const Schedule* s) {
     if (adjoint || nsamples == 1) return s->nsamples == nsamples;
     return s->nsamples > 1 && s->nsamples >= nsamples;
   };
   for (Schedule* s : c->scheds)
-    if (s->N == N && s->dm == dm && !s->dagger && s->t == tu.t && s->asked == tu.R && fits(s) &&
+    if (s->N == N && s->dm == dm && !s->dagger && s->t == tu.t && s->asked == asked && fits(s) &&
         (adjoint || s->fuse == (tu.fuse != 0)) &&
         s->lo == lo && s->hi == hi && s->adjoint == adjoint && s->tile_only == tile_only) {
       *out = s;
@@ -2122,7 +2123,8 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
   S->N = N;
   S->dm = dm;
   S->t = tu.t;
-  S->R = S->asked = tu.R;
+  S->R = tu.R;
+  S->asked = asked;
   S->nsamples = nsamples;
   S->lo = lo;
   S->hi = hi;
@@ -2222,33 +2224,23 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
     dev_free(S->d_frecs);
     dev_free(S->d_fcomps);
   };
-  if (!adjoint && !tile_only && tu.strict) {
-    S->strict = true;
+  // Fallbacks belong to the schedule: it keeps the width it stands for (asked), and other circuits of the
+  // size choose theirs afresh. Width 4 taken by size needs every specialised kernel, else width 3 does,
+  // whose sources are shorter; width 3 exists only as specialised kernels, so where they cannot
+  // all be built (source limits, compile budget) width 4 runs partly interpreted. (A width forced through
+  // MB_REG_BITS is kept; run_schedule then reports the missing kernels. Tile-only schedules belong
+  // to the persistent uneven launch, which compiles its own kernel.)
+  if (!adjoint && !tile_only && (tu.strict || (S->R == 3 && !getenv("MB_REG_BITS")))) {
+    S->strict = tu.strict;
     prepare_jit(S.get());
     if (S->jit != 1) {
+      Tuning other = tu;
+      other.R = tu.strict ? 3 : 4;
+      other.asked = asked;
+      if (getenv("MB_JIT_VERBOSE"))
+        fprintf(stderr, "mossb200: a %d-bit schedule falls back from register width %d to %d\n", N, S->R, other.R);
       drop();
-      Tuning three = tu;
-      three.R = 3;
-      const int rc3 = get_schedule_impl(c, n, dm, adjoint, lo, hi, nsamples, &three, tile_only, out);
-      if (rc3 == MB_OK && (*out)->R == 3) (*out)->asked = 4;
-      return rc3;
-    }
-  }
-  if (!adjoint && !tile_only && S->R == 3 && !getenv("MB_REG_BITS")) {
-    // Register width 3 exists only as specialised kernels: if they cannot all be built (source
-    // limits, compile budget), use width 4 for this register size from now on. (A width forced
-    // through MB_REG_BITS is kept; run_schedule then reports the missing kernels. Tile-only
-    // schedules belong to the persistent uneven launch, which compiles its own kernel.)
-    prepare_jit(S.get());
-    if (S->jit != 1) {
-      if (getenv("MB_JIT_VERBOSE")) fprintf(stderr, "mossb200: %d-bit schedules fall back to register width 4\n", N);
-      {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        g_tuning[N] = {S->t, 4};
-        g_partial.insert(N);
-      }
-      drop();
-      return get_schedule_impl(c, n, dm, adjoint, lo, hi, nsamples, nullptr, tile_only, out);
+      return get_schedule_impl(c, n, dm, adjoint, lo, hi, nsamples, &other, tile_only, out);
     }
   }
   *out = S.get();
@@ -2659,6 +2651,23 @@ int apply_fused(mb_circuit c, mb_state s, int64_t mrow_stride) {
   int rc = get_schedule(c, s->n, dm, false, s->batch, &S);
   if (rc) return rc;
   return run_schedule(c, S, s->d, s->batch, mrow_stride);
+}
+
+// Tile bits and register width that circuit c runs with on s once scheduled (the tuned ones where it
+// runs without a schedule).
+int schedule_widths(mb_circuit c, mb_state s, int* t, int* R) {
+  const int dm = s->kind == MB_DENSITY || s->kind == MB_BATCH_DENSITY, N = dm ? 2 * s->n : s->n;
+  const Tuning tu = tuning_for(N);
+  *t = tu.t;
+  *R = tu.R;
+  if (N < 8) return MB_OK;
+  for (const COp& op : c->ops)
+    if (op.kind == MB_OP_GATE && op.k == 0) return MB_OK;
+  Schedule* S = nullptr;
+  if (int rc = get_schedule(c, s->n, dm, false, s->batch, &S)) return rc;
+  *t = S->t;
+  *R = S->R;
+  return MB_OK;
 }
 
 void release_schedules(mb_circuit c) {

@@ -161,8 +161,8 @@ extern "C" int mb_autotune(mb_circuit c, mb_state s, const double* theta, size_t
       return true;
     }
     int et = 0, er = 0;
-    mb_tuning_get(N, &et, &er);
-    if (et != cd[0] || er != cd[1]) return true;  // the library fell back to another width
+    if ((rc = schedule_widths(c, s, &et, &er))) return false;
+    if (et != cd[0] || er != cd[1]) return true;  // the schedule fell back to another width
     cudaEventRecord(a, g_ctx.stream);
     for (int k = 0; k < 2 && !rc; ++k) rc = mb_apply(c, s, theta, ntheta, flags & ~MB_APPLY_PLAIN);
     cudaEventRecord(b, g_ctx.stream);
