@@ -2369,16 +2369,12 @@ static void prepare_jit(Schedule* S) {
   }
   std::vector<CUfunction> fns;
   std::string err;
-  // Passes whose kernels do not compile within the budget (MB_JIT_BUDGET_S seconds per
-  // schedule, default 30), and passes whose generated source exceeds MB_JIT_MAX_SOURCE_KB
-  // (default 128 KB; NVRTC time grows faster than the source: 3 s at 97 KB, 17 s at 238 KB), run on the
-  // interpreter kernels, which exist for R = 4 and 5; the adjoint and R = 3 schedules need
+  // Passes whose kernels do not compile within the budget, and passes whose generated source exceeds the
+  // limit, run on the interpreter kernels, which exist for R = 4 and 5; the adjoint and R = 3 schedules need
   // every specialised kernel (an R = 3 schedule that cannot have them is rebuilt with R = 4;
   // the adjoint's size limit is four times larger).
-  double budget = 30.0;
-  if (const char* e = getenv("MB_JIT_BUDGET_S")) budget = atof(e);
-  size_t max_src = size_t(128) << 10;
-  if (const char* e = getenv("MB_JIT_MAX_SOURCE_KB")) max_src = size_t(std::max(1, atoi(e))) << 10;
+  const double budget = jit_budget_s();
+  size_t max_src = jit_max_source();
   const bool partial_ok = !S->adjoint && (S->R == 4 || S->R == 5) && !S->strict;
   if (S->adjoint) max_src *= 4;  // no interpreter to fall back on: only refuse the extreme ones
   std::vector<std::string> small;

@@ -1819,6 +1819,28 @@ int jit_prepare(std::vector<std::string>& sources, std::vector<CUfunction>& out,
   return MB_OK;
 }
 
+bool jit_cached(const std::vector<std::string>& sources, std::vector<CUfunction>& out) {
+  out.assign(sources.size(), nullptr);
+  std::lock_guard<std::mutex> lk(g_jit_mu);
+  for (size_t i = 0; i < sources.size(); ++i) {
+    auto it = g_cache.find(sources[i]);
+    if (it == g_cache.end()) return false;
+    out[i] = it->second.fn;
+    it->second.last = ++g_tick;
+  }
+  return true;
+}
+
+size_t jit_max_source() {
+  const char* e = getenv("MB_JIT_MAX_SOURCE_KB");
+  return size_t(e ? std::max(1, atoi(e)) : 128) << 10;
+}
+
+double jit_budget_s() {
+  const char* e = getenv("MB_JIT_BUDGET_S");
+  return e ? atof(e) : 30.0;
+}
+
 int jit_launch_tile(CUfunction fn, const CUtensorMap* map, const double2* tab, const double2* xtab, const double2* xtabs,
                     int64_t xrow, int64_t tstride, int64_t tps, int64_t ntiles, unsigned* err, int threads, size_t shm,
                     int grid, cudaStream_t st) {

@@ -26,6 +26,13 @@ std::string jit_reg_source(const Pass& p, int N, bool stage_params);
 // the call still succeeds; a source that fails to compile always fails the call.
 int jit_prepare(std::vector<std::string>& sources, std::vector<CUfunction>& out, std::string* err,
                 double budget_s = 0);
+// Takes every source's kernel from the cache; false (and nothing taken) when one is missing.
+bool jit_cached(const std::vector<std::string>& sources, std::vector<CUfunction>& out);
+// Limits of generated kernels: the bytes of a source (MB_JIT_MAX_SOURCE_KB, default 128 KB; NVRTC time
+// grows faster than the source: 3 s at 97 KB, 17 s at 238 KB) and the seconds within which the sources of a
+// schedule or observable have to start compiling (MB_JIT_BUDGET_S, default 30).
+size_t jit_max_source();
+double jit_budget_s();
 int jit_launch_tile(CUfunction fn, const CUtensorMap* map, const double2* tab, const double2* xtab, const double2* xtabs,
                     int64_t xrow, int64_t tstride, int64_t tps, int64_t ntiles, unsigned* err, int threads, size_t shm,
                     int grid, cudaStream_t st);

@@ -74,6 +74,8 @@ struct PauliProgram {
   double2* d_coef = nullptr;     // the observable's string coefficients, for the specialised kernels
   int psum_t = 0;                // tile bits of the staged passes, when the program has them
   std::vector<void*> psum;       // staged expectation kernels (mbk_psum), one per pass
+  bool waiting = false;          // they are compiled once the program is used again
+  int uses = 0;                  // expectations so far, while waiting
 };
 
 struct PauliData {
@@ -641,20 +643,25 @@ static int pauli_coefficients(PauliData* pd, PauliProgram* P) {
   return MB_OK;
 }
 
-// Compiles the staged passes of a program; false leaves it as it was (no placement, no compiler,
-// or a kernel that spills).
-static bool pauli_stage(PauliData* pd, PauliProgram* P) {
+// Takes the staged passes of a program, compiling them within the limits of every generated kernel (source
+// length, seconds per program) or, without `compile`, only if their kernels are there already. False leaves
+// the program as it was (no placement, no compiler, past a limit, or a kernel that spills).
+static bool pauli_stage(PauliData* pd, PauliProgram* P, bool compile) {
   const std::vector<PsumPass> plan = psum_plan(pd, P->n);
   if (plan.empty()) return false;
   std::vector<std::string> src;
   for (const PsumPass& p : plan) {
     src.push_back(jit_psum_source(p));
-    if (src.back().empty() || src.back().size() > (size_t(256) << 10)) return false;
+    if (src.back().empty() || src.back().size() > jit_max_source()) return false;
   }
-  if (pauli_coefficients(pd, P) != MB_OK) return false;
   std::vector<CUfunction> fns;
   std::string err;
-  if (jit_prepare(src, fns, &err, 0.0) != MB_OK) {
+  if (!compile && !jit_cached(src, fns)) {
+    P->waiting = true;
+    return false;
+  }
+  if (pauli_coefficients(pd, P) != MB_OK) return false;
+  if (compile && jit_prepare(src, fns, &err, jit_budget_s()) != MB_OK) {
     if (getenv("MB_JIT_VERBOSE")) fprintf(stderr, "mossb200: staged Pauli passes: %s\n", err.c_str());
     return false;
   }
@@ -670,7 +677,10 @@ static bool pauli_stage(PauliData* pd, PauliProgram* P) {
 
 // Specialised kernels for a program from MB_PAULI_JIT_MIN_BITS qubits (default 14; MB_PAULI_JIT=0
 // disables them): the staged passes where every flip mask fits a tile and no kernel spills, else one
-// mbk_pauli per pass (MB_PAULI_STAGED=0 goes straight to those). A pass whose per-thread factors would take too
+// mbk_pauli per pass (MB_PAULI_STAGED=0 goes straight to those). Programs of wide tiles (from 24 qubits), which
+// have no mbk_pauli, run interpreted until their second expectation unless the staged kernels are there: compiling
+// them takes 0.2 to 0.6 s, the interpreter 1 to 30 ms, so an observable used once would pay a hundredfold
+// (26 qubits, XXZ: first call 7 against 213 ms, later ones 4.6 against 0.64). A pass whose per-thread factors would take too
 // many registers, or whose kernel does not compile, keeps the interpreter kernel, and so do
 // programs built on a thread that may not compile (the serving loop: a request's observable
 // is often new, and neither NVRTC nor the source generation belongs on its path).
@@ -681,7 +691,7 @@ static void pauli_specialise(PauliData* pd, PauliProgram* P, const std::vector<P
   const char* e = getenv("MB_PAULI_JIT");
   if ((e && atoi(e) == 0) || P->n < min_bits || !t_pauli_compile || !jit_available() || pd->strings.empty()) return;
   const char* staged = getenv("MB_PAULI_STAGED");
-  if (!(staged && atoi(staged) == 0) && pauli_stage(pd, P)) return;
+  if (!(staged && atoi(staged) == 0) && pauli_stage(pd, P, P->nr <= 5)) return;
   std::vector<std::string> src;
   std::vector<size_t> which;
   // Passes of 2^12-amplitude tiles (from 24 qubits) keep the interpreter unless
@@ -882,6 +892,7 @@ bool pauli_usable(mb_observable o, mb_state s) {
 }
 
 int expect_pauli(mb_observable o, mb_state s, double2* out) {
+  const bool prepared = out != nullptr;
   if (!out) out = g_ctx.results;
   PauliProgram* P = nullptr;
   if (g_ctx.capturing) {
@@ -894,6 +905,11 @@ int expect_pauli(mb_observable o, mb_state s, double2* out) {
   } else {
     int rc = pauli_program(o, s->n, &P);
     if (rc) return rc;
+    // results that stay on the device are those of a prepared plan, which is recorded next
+    if (P && P->waiting && t_pauli_compile && (prepared || ++P->uses > 1)) {
+      P->waiting = false;
+      pauli_stage(o->pauli, P, true);
+    }
   }
   if (!P) return expect_keys(o, s, out);
   cudaStream_t st = g_ctx.stream;
