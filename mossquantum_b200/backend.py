@@ -102,8 +102,9 @@ def apply_(operation, state, theta=None, plain=False, tensor=False):
     if not isinstance(state, _DeviceState):
         raise TypeError("apply_ needs a B200 state")
     circuit = _as_circuit(operation) if isinstance(operation, (Gate, QCircuit)) else None
-    key = circuit.value_key() if circuit is not None else None
-    known = circuit.known(state.n, key) if circuit is not None else None
+    # a circuit that is new on this size has nothing to be recognised by
+    key = circuit.value_key() if circuit is not None and circuit.seen(state.n) else None
+    known = circuit.known(state.n, key) if key is not None else None
     if known is not None:
         # these values passed the checks below on an earlier call
         compiled, has_channel = known
@@ -123,6 +124,7 @@ def apply_(operation, state, theta=None, plain=False, tensor=False):
             _validate_positions(operation, state.n)
             if circuit is None:
                 circuit = _as_circuit(operation)
+            if key is None:
                 key = circuit.value_key()
             if circuit.has_channel() and not state.is_density:
                 state = density_of(state)
