@@ -733,24 +733,43 @@ int theta_check(mb_circuit c, const double* theta, size_t ntheta, int rows) {
   return MB_OK;
 }
 
-int small_reserve(size_t host_doubles, size_t device_doubles) {
-  if (host_doubles + 2 > g_ctx.h_small_cap) {
-    const size_t cap = std::max<size_t>(2 * host_doubles, 4096);
-    double* p = nullptr;
-    MB_CHECK_CUDA(cudaMallocHost((void**)&p, sizeof(double) * cap));
-    if (g_ctx.h_small) cudaFreeHost(g_ctx.h_small);
-    g_ctx.h_small = p;
-    g_ctx.h_small_cap = cap;
+int SmallBufs::take(size_t host_doubles, size_t device_doubles) {
+  // two more for alignment
+  const size_t hn = host_doubles + 2, dn = device_doubles + 2;
+  if (hn > kSmallKeep) {
+    MB_CHECK_CUDA(cudaMallocHost((void**)&h_own, sizeof(double) * hn));
+    h = h_own;
+  } else {
+    if (hn > g_ctx.h_small_cap) {
+      const size_t cap = std::min(kSmallKeep, std::max<size_t>(2 * hn, 4096));
+      double* p = nullptr;
+      MB_CHECK_CUDA(cudaMallocHost((void**)&p, sizeof(double) * cap));
+      if (g_ctx.h_small) cudaFreeHost(g_ctx.h_small);
+      g_ctx.h_small = p;
+      g_ctx.h_small_cap = cap;
+    }
+    h = g_ctx.h_small;
   }
-  if (device_doubles + 2 > g_ctx.d_small_cap) {
-    const size_t cap = std::max<size_t>(2 * device_doubles, 4096);
-    double* p = nullptr;
-    if (int rc = dev_alloc((void**)&p, sizeof(double) * cap)) return rc;
-    dev_free(g_ctx.d_small);
-    g_ctx.d_small = p;
-    g_ctx.d_small_cap = cap;
+  if (dn > kSmallKeep) {
+    if (int rc = dev_alloc((void**)&d_own, sizeof(double) * dn)) return rc;
+    d = d_own;
+  } else {
+    if (dn > g_ctx.d_small_cap) {
+      const size_t cap = std::min(kSmallKeep, std::max<size_t>(2 * dn, 4096));
+      double* p = nullptr;
+      if (int rc = dev_alloc((void**)&p, sizeof(double) * cap)) return rc;
+      dev_free(g_ctx.d_small);
+      g_ctx.d_small = p;
+      g_ctx.d_small_cap = cap;
+    }
+    d = g_ctx.d_small;
   }
   return MB_OK;
+}
+
+SmallBufs::~SmallBufs() {
+  if (h_own) cudaFreeHost(h_own);
+  dev_free(d_own);
 }
 
 // Validates theta and stages it into the circuit's device parameter buffer (asynchronously,

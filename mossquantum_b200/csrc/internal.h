@@ -94,6 +94,7 @@ struct mb_observable_s {
 namespace mb {
 
 constexpr size_t kThetaStage = size_t(1) << 20;
+constexpr size_t kSmallKeep = size_t(1) << 20;   // doubles kept for small synchronous calls: 8 MiB
 
 struct Ctx {
   bool init = false;
@@ -141,9 +142,19 @@ int bind_circuit(mb_circuit c, const double* theta, size_t ntheta, int rows);
 int theta_stage(mb_circuit c, const double* theta, size_t ntheta, int rows);
 int bind_launch(mb_circuit c, int rows);
 int theta_check(mb_circuit c, const double* theta, size_t ntheta, int rows);
-// Room for so many doubles in h_small / d_small (and two more for alignment). Only for calls that
-// hold the library lock until their copies have finished.
-int small_reserve(size_t host_doubles, size_t device_doubles);
+// Pinned and device memory for so many doubles: h_small and d_small up to kSmallKeep, else memory of the
+// call's own. Only for calls that hold the library lock until their copies have finished.
+struct SmallBufs {
+  double *h = nullptr, *d = nullptr;
+  int take(size_t host_doubles, size_t device_doubles);
+  ~SmallBufs();
+  SmallBufs() = default;
+  SmallBufs(const SmallBufs&) = delete;
+  SmallBufs& operator=(const SmallBufs&) = delete;
+
+ private:
+  double *h_own = nullptr, *d_own = nullptr;
+};
 // Target local bit of a fixed matrix that is the identity unless every other bit is 1, or -1.
 int controlled_target(const double2* M, int k);
 int check_not_capturing(const char* what);

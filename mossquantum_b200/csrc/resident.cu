@@ -894,9 +894,10 @@ int resident_run(mb_circuit c, mb_observable o, mb_state init, const double* the
   // are free again when it returns.
   const size_t ns = size_t(c->nslots), nw = grad ? size_t(B) : 0;
   const size_t down = 2 * size_t(B) + (grad ? ns : 0), rows = grad && B > 1 ? size_t(B) * ns : 0;
-  if (int rc = small_reserve(ns + nw + down, ns + nw + rows)) return rc;
-  double* hp = g_ctx.h_small;
-  double* dp = g_ctx.d_small;
+  SmallBufs bufs;
+  if (bufs.take(ns + nw + down, ns + nw + rows)) return MB_OK;   // no room: the general form
+  double* hp = bufs.h;
+  double* dp = bufs.d;
   RTheta th;
   const bool direct = ns <= kResTheta;
   std::copy(theta, theta + ns, direct ? th.v : hp);
@@ -935,7 +936,7 @@ int resident_run(mb_circuit c, mb_observable o, mb_state init, const double* the
   a.init = init->d;
   a.flips = os.flips;
   a.strings = os.strings;
-  double* res = hp + ns + nw + ((ns + nw) & 1);   // 16-byte aligned; small_reserve leaves room
+  double* res = hp + ns + nw + ((ns + nw) & 1);   // 16-byte aligned; the buffer leaves room
   a.values = reinterpret_cast<double2*>(res);
   a.gout = res + 2 * size_t(B);
   a.gsample = dp + ns + nw;
