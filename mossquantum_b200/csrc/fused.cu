@@ -463,6 +463,15 @@ struct AccRec {
 };
 
 struct Schedule {
+  Schedule() = default;
+  Schedule(const Schedule&) = delete;
+  Schedule& operator=(const Schedule&) = delete;
+  // (also for a schedule that ran out of memory while it was built)
+  ~Schedule() {
+    for (void* p : {(void*)d_accs, (void*)d_run_mats, (void*)d_xtab, (void*)d_fcomps, (void*)d_frecs, (void*)d_gslots,
+                    (void*)d_stages, (void*)d_mops})
+      dev_free(p);
+  }
   std::vector<std::vector<int>> runs;   // instructions of each fused run, in the order of undoing
   std::vector<AccRec> accs;
   std::vector<int> run_mats;            // table offsets of the runs' gate matrices
@@ -2216,14 +2225,6 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
                                     cudaMemcpyHostToDevice, g_ctx.stream));
   }
   MB_CHECK_CUDA(cudaStreamSynchronize(g_ctx.stream));
-  auto drop = [&] {
-    dev_free(S->d_stages);
-    dev_free(S->d_mops);
-    dev_free(S->d_gslots);
-    dev_free(S->d_xtab);
-    dev_free(S->d_frecs);
-    dev_free(S->d_fcomps);
-  };
   // Fallbacks belong to the schedule: it keeps the width it stands for (asked), and other circuits of the
   // size choose theirs afresh. Width 4 taken by size needs every specialised kernel, else width 3 does,
   // whose sources are shorter; width 3 exists only as specialised kernels, so where they cannot
@@ -2239,7 +2240,7 @@ static int get_schedule_impl(mb_circuit c, int n, int dm, int adjoint, int lo, i
       other.asked = asked;
       if (getenv("MB_JIT_VERBOSE"))
         fprintf(stderr, "mossb200: a %d-bit schedule falls back from register width %d to %d\n", N, S->R, other.R);
-      drop();
+      S.reset();
       return get_schedule_impl(c, n, dm, adjoint, lo, hi, nsamples, &other, tile_only, out);
     }
   }
@@ -2670,14 +2671,6 @@ void release_schedules(mb_circuit c) {
   for (Schedule* s : c->scheds) {
     for (const Pass& p : s->passes)
       if (p.jit_fn) jit_release(p.jit_fn);
-    dev_free(s->d_stages);
-    dev_free(s->d_mops);
-    dev_free(s->d_gslots);
-    dev_free(s->d_xtab);
-    dev_free(s->d_frecs);
-    dev_free(s->d_fcomps);
-    dev_free(s->d_accs);
-    dev_free(s->d_run_mats);
     delete s;
   }
   c->scheds.clear();
