@@ -2566,21 +2566,19 @@ int run_adjoint_schedule(mb_circuit c, Schedule* S, double2* y, double2* d, doub
     set_error("state too small for the fused adjoint");
     return MB_EUNSUPPORTED;
   }
-  double* gpart = nullptr;
-  double* acc = nullptr;
-  unsigned* gcount = nullptr;
+  struct Mem {
+    void* p = nullptr;
+    ~Mem() { dev_free(p); }
+  } mpart, mcount, macc;
   const int grid_max = g_ctx.sm_count * 4;
   int rc;
-  if ((rc = dev_alloc((void**)&gpart, sizeof(double) * std::max(1, S->max_grad) * grid_max))) return rc;
-  if ((rc = dev_alloc((void**)&gcount, sizeof(unsigned)))) {
-    dev_free(gpart);
+  if ((rc = dev_alloc(&mpart.p, sizeof(double) * std::max(1, S->max_grad) * grid_max)) ||
+      (rc = dev_alloc(&mcount.p, sizeof(unsigned))) ||
+      (rc = dev_alloc(&macc.p, sizeof(double) * std::max(1, S->nacc))))
     return rc;
-  }
-  if ((rc = dev_alloc((void**)&acc, sizeof(double) * std::max(1, S->nacc)))) {
-    dev_free(gpart);
-    dev_free(gcount);
-    return rc;
-  }
+  double* gpart = static_cast<double*>(mpart.p);
+  double* acc = static_cast<double*>(macc.p);
+  unsigned* gcount = static_cast<unsigned*>(mcount.p);
   cudaMemsetAsync(gcount, 0, sizeof(unsigned), st);
   const int B = S->nsamples;
   double2* xs = S->d_xtab ? S->d_xtab + S->xtab.size() : nullptr;
@@ -2617,9 +2615,6 @@ int run_adjoint_schedule(mb_circuit c, Schedule* S, double2* y, double2* d, doub
       rc = MB_EDEVICE;
     }
   }
-  dev_free(acc);
-  dev_free(gpart);
-  dev_free(gcount);
   return rc;
 }
 
