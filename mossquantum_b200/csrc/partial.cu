@@ -71,6 +71,30 @@ __global__ void __launch_bounds__(256) k_partial_trace_dm(const double2* __restr
   }
 }
 
+// Pure states, few traced configurations and few products: one thread per entry of r. The staged product
+// below takes 4 to 10 us more to start: 4 qubits, 2 kept 21 against 31 us a call, 8 qubits, 4 kept 26
+// against 30, 12 qubits, 8 kept 28 against 34. Beyond 2^20 products (12 qubits, 10 kept: 44 against
+// 30) or 2^4 terms per thread (2^5 from six kept qubits; 8 qubits, 2 kept, 2^6 terms: 42 against 32) it is faster.
+constexpr int64_t kPTFewWork = int64_t(1) << 20;
+__global__ void __launch_bounds__(256) k_partial_entries(const double2* __restrict__ in, double2* __restrict__ out, int n,
+                                                         const Split sp, int nsamples) {
+  const int64_t total = int64_t(nsamples) << (2 * sp.m), dm_out = int64_t(1) << sp.m;
+  const int nt = 1 << sp.k;
+  for (int64_t g = int64_t(blockIdx.x) * 256 + threadIdx.x; g < total; g += int64_t(gridDim.x) * 256) {
+    const double2* s = in + ((g >> (2 * sp.m)) << n);
+    const int64_t ra = deposit(g & (dm_out - 1), sp.m, sp.keep), rc = deposit((g >> sp.m) & (dm_out - 1), sp.m, sp.keep);
+    double re = 0.0, im = 0.0;
+#pragma unroll 4
+    for (int t = 0; t < nt; ++t) {
+      const int64_t rt = deposit(t, sp.k, sp.trace);
+      const double2 u = s[ra | rt], v = s[rc | rt];   // u * conj(v)
+      re += u.x * v.x + u.y * v.y;
+      im += u.y * v.x - u.x * v.y;
+    }
+    out[g] = make_double2(re, im);
+  }
+}
+
 // Pure states: r = V V', V[a, t] = psi[(a, t)], as a blocked product. A CTA owns one pair of
 // 2^ma-row blocks (ma = min(m, 6)) of r and one chunk of t; per step it stages both blocks' tiles of
 // 2^tb columns (2^(ma + tb) <= 2^11 amplitudes) with cp.async, double-buffered, the copy running
@@ -374,6 +398,7 @@ int trace_pure_bs(mb_state in, TraceArgs a, mb_state out) {
     const double2* src = in->d + (int64_t(b0) << a.n);
     double2* dst = out->d + (int64_t(b0) << (2 * a.m));
     double2* pt = part ? part + per * b0 : nullptr;
+    ProfScope ps("k_partial_outer", 16.0 * double(int64_t(1) << a.n) * nbat, g_ctx.stream);
     outer<<<dim3(a.npairs, a.chunks, nbat), nt, shm, g_ctx.stream>>>(src, a, pt, dst);
     ++launch_counter();
     if (a.chunks > 1) {
@@ -395,6 +420,13 @@ int trace_pure_bs(mb_state in, TraceArgs a, mb_state out) {
 }
 
 int trace_pure(mb_state in, const Split& sp, mb_state out) {
+  const int64_t entries = int64_t(in->batch) << (2 * sp.m);
+  if (sp.k <= (sp.m >= 6 ? 5 : 4) && entries <= (kPTFewWork >> sp.k)) {
+    ProfScope ps("k_partial_entries", 16.0 * double(in->elems) * in->batch, g_ctx.stream);
+    k_partial_entries<<<grid_for(entries, 256), 256, 0, g_ctx.stream>>>(in->d, out->d, in->n, sp, in->batch);
+    MB_LAUNCHED();
+    return MB_OK;
+  }
   TraceArgs a{};
   a.n = in->n;
   a.m = sp.m;
