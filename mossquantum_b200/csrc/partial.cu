@@ -37,16 +37,16 @@ __host__ __device__ __forceinline__ int64_t deposit(int64_t x, int nb, const int
 template <int L>
 __global__ void __launch_bounds__(256) k_partial_trace_dm(const double2* __restrict__ in, double2* __restrict__ out,
                                                           int n, const Split sp, int nsamples) {
-  const int64_t dm_out = int64_t(1) << sp.m, per = dm_out * dm_out, total = per * nsamples;
-  const int64_t dim = int64_t(1) << n, nt = int64_t(1) << sp.k;
+  const int64_t dm_out = int64_t(1) << sp.m, total = int64_t(nsamples) << (2 * sp.m);
+  const int64_t dim = int64_t(1) << n;
+  const int nt = 1 << sp.k;
   __shared__ double2 part[8];
   const int sub = threadIdx.x & (L - 1);
   for (int64_t g = (int64_t(blockIdx.x) * 256 + threadIdx.x) / L; g < total; g += int64_t(gridDim.x) * 256 / L) {
-    const int64_t b = g / per, e = g - b * per;
-    const double2* s = in + b * dim * dim +
-                       (deposit(e % dm_out, sp.m, sp.keep) + deposit(e / dm_out, sp.m, sp.keep) * dim);
+    const double2* s = in + ((g >> (2 * sp.m)) << (2 * n)) +
+                       (deposit(g & (dm_out - 1), sp.m, sp.keep) + deposit((g >> sp.m) & (dm_out - 1), sp.m, sp.keep) * dim);
     double re = 0.0, im = 0.0;
-    for (int64_t t = sub; t < nt; t += L) {
+    for (int t = sub; t < nt; t += L) {
       const double2 x = s[deposit(t, sp.k, sp.trace) * (dim + 1)];
       re += x.x;
       im += x.y;
