@@ -13,6 +13,7 @@
 // accesses whenever the gate bits are not the lowest ones.
 #include <algorithm>
 #include <cstdarg>
+#include <type_traits>
 
 #include "family.cuh"
 #include "kernels.h"
@@ -375,8 +376,8 @@ __global__ void k_obs_scalar(const double2* __restrict__ in, double2* __restrict
 // in unread bits added (shuffles) and the bins written, each by one lane: no contention however
 // few the bins, and the same sum on every run. With splits > 1 the units write partial
 // histograms that k_marginal_sum adds in order.
-// Bound: one read of the state (HBM, or L2 up to about 2^22 amplitudes). Ten of 22 qubits: 16 us
-// and 4 us for the sum, against 36 us with a shared-memory histogram and double atomics.
+// Bound: one read of the state (HBM, or L2 up to about 2^22 amplitudes). Ten of 22 qubits: 12.7 us
+// and 6.6 us for the sum, against 70 us with a shared-memory histogram and double atomics.
 struct Readout {
   int nq;
   int nh;                 // readout bits above the lanes
@@ -393,6 +394,7 @@ __device__ __forceinline__ uint64_t deposit_mask(uint64_t x, uint64_t mask) {
   return r;
 }
 
+constexpr int kMarginalTerms = 16;   // loads in flight per lane
 template <bool DM>
 __global__ void __launch_bounds__(kBlock) k_marginal(const double2* __restrict__ v, int n, const Readout ro, int splits,
                                                       int nsamples, double* out, unsigned* flags, double tol) {
@@ -417,16 +419,16 @@ __global__ void __launch_bounds__(kBlock) k_marginal(const double2* __restrict__
     double p = 0.0;
     if (lane < dim) {
       uint64_t x = deposit_mask(uint64_t(s) * per, ro.inner);
-      int64_t i = 0;
-      for (; i + 4 <= per; i += 4) {
-        double2 a[4];
+      auto terms = [&](auto width) {   // so many loads in flight
+        constexpr int W = decltype(width)::value;
+        double2 a[W];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < W; ++k) {
           a[k] = vs[int64_t(base | x) * stride];
           x = ((x | ~ro.inner) + 1) & ro.inner;
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
+        for (int k = 0; k < W; ++k) {
           if (DM) {
             bad |= (fabs(a[k].y) > tol ? 1u : 0u) | (a[k].x < -tol ? 2u : 0u);
             p += a[k].x;
@@ -434,17 +436,10 @@ __global__ void __launch_bounds__(kBlock) k_marginal(const double2* __restrict__
             p += a[k].x * a[k].x + a[k].y * a[k].y;
           }
         }
-      }
-      for (; i < per; ++i) {
-        const double2 a = vs[int64_t(base | x) * stride];
-        x = ((x | ~ro.inner) + 1) & ro.inner;
-        if (DM) {
-          bad |= (fabs(a.y) > tol ? 1u : 0u) | (a.x < -tol ? 2u : 0u);
-          p += a.x;
-        } else {
-          p += a.x * a.x + a.y * a.y;
-        }
-      }
+      };
+      int64_t i = 0;
+      for (; i + kMarginalTerms <= per; i += kMarginalTerms) terms(std::integral_constant<int, kMarginalTerms>());
+      for (; i < per; ++i) terms(std::integral_constant<int, 1>());
     }
     bool mine = lane < dim;
 #pragma unroll
@@ -465,17 +460,27 @@ __global__ void __launch_bounds__(kBlock) k_marginal(const double2* __restrict__
   }
 }
 
+// Adds the parts of every bin in a fixed order: L threads (a warp, or a block where bins are few and
+// parts many) stride over them, then a butterfly and the warps in order.
+template <int L>
 __global__ void __launch_bounds__(kBlock) k_marginal_sum(const double* __restrict__ part, int splits, int64_t count,
                                                           double* __restrict__ out) {
-  // one warp per bin: lanes over the splits, then a fixed butterfly
-  const int lane = threadIdx.x & 31;
-  for (int64_t i = int64_t(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5); i < count;
-       i += int64_t(gridDim.x) * (kBlock / 32)) {
+  __shared__ double warp_sum[kBlock / 32];
+  const int sub = threadIdx.x & (L - 1);
+  for (int64_t i = (int64_t(blockIdx.x) * kBlock + threadIdx.x) / L; i < count; i += int64_t(gridDim.x) * kBlock / L) {
     double p = 0.0;
-    for (int s = lane; s < splits; s += 32) p += part[int64_t(s) * count + i];
+#pragma unroll 8
+    for (int s = sub; s < splits; s += L) p += part[int64_t(s) * count + i];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
-    if (lane == 0) out[i] = p;
+    if (L > 32) {
+      if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = p;
+      __syncthreads();
+      if (sub == 0)
+        for (int w = 1; w < L / 32; ++w) p += warp_sum[w];
+      __syncthreads();
+    }
+    if (sub == 0) out[i] = p;
   }
 }
 
@@ -675,11 +680,12 @@ int launch_marginal(const double2* v, int n, int is_dm, int nsamples, const int*
     if (q < 5) ro.lbin[q] = j;
     else ro.hpos[ro.nh] = q, ro.hbin[ro.nh++] = j;
   }
-  // Split the sums while the units leave warps idle (64 warps per SM wanted), a part keeps at
-  // least 16 terms per lane, and the partial histograms fit the scratch.
+  // Split the sums while the units leave warps idle (16 per SM are enough at 16 loads in flight; 64 with
+  // 22 qubits, one read: 62 us a call against 50), a part keeps at least 4 terms per lane (16 qubits, one read:
+  // 7.0 us of kernel, 8.1 with parts of 16), and the partial histograms fit the scratch.
   const int64_t count = (int64_t(1) << nq) * nsamples;
   int splits = 1;
-  while ((int64_t(nsamples) * splits << ro.nh) < int64_t(148) * 64 && (int64_t(1) << ro.ninner) / splits >= 32 &&
+  while ((int64_t(nsamples) * splits << ro.nh) < int64_t(148) * 16 && (int64_t(1) << ro.ninner) / splits >= 8 &&
          int64_t(splits) * 2 * count <= scratch_cap)
     splits *= 2;
   const int64_t units = (int64_t(nsamples) * splits) << ro.nh;
@@ -693,7 +699,9 @@ int launch_marginal(const double2* v, int n, int is_dm, int nsamples, const int*
   }
   MB_LAUNCHED();
   if (splits > 1) {
-    k_marginal_sum<<<grid_for(count, kBlock / 32, int64_t(148) * 8), kBlock, 0, st>>>(scratch, splits, count, out);
+    const int64_t cap = int64_t(148) * 8;
+    if (splits >= kBlock && count <= cap) k_marginal_sum<kBlock><<<grid_for(count, 1, cap), kBlock, 0, st>>>(scratch, splits, count, out);
+    else k_marginal_sum<32><<<grid_for(count, kBlock / 32, cap), kBlock, 0, st>>>(scratch, splits, count, out);
     MB_LAUNCHED();
   }
   return MB_OK;
