@@ -203,13 +203,14 @@ int resident_run(mb_circuit c, mb_observable o, mb_state init, const double* the
 void resident_release(mb_circuit c);
 
 // pauli.cu
-// The observable's strings on the device; false when one acts outside n qubits.
+// The observable's strings on the device; false when one acts outside n qubits, when they are more than
+// `most`, or when they cannot be put there.
 struct ObsStrings {
   const PFlip* flips = nullptr;
   const PString* strings = nullptr;
   int nflips = 0, nstr = 0;
 };
-bool observable_strings(mb_observable o, int n, ObsStrings* out);
+bool observable_strings(mb_observable o, int n, int64_t most, ObsStrings* out);
 int pauli_compile(mb_observable o, const mb_term* terms, size_t nterms);
 void pauli_free(mb_observable o);
 int expect_pauli(mb_observable o, mb_state s, double2* out = nullptr);

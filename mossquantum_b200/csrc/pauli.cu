@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <complex>
 #include <map>
 #include <memory>
@@ -82,8 +83,8 @@ struct PauliData {
   std::vector<PString> strings;  // grouped by flip mask
   std::vector<std::pair<uint64_t, std::pair<int, int>>> groups;  // x -> [s0, ns)
   std::vector<PauliProgram*> programs;
-  PFlip* d_flips = nullptr;      // groups and strings on the device (density matrices)
-  PString* d_all = nullptr;
+  PString* d_all = nullptr;      // strings, then groups, on the device (density matrices, small states)
+  PFlip* d_flips = nullptr;
   int64_t dense_rows = 0;        // sum over the site keys of their matrix dimension
 };
 
@@ -429,29 +430,42 @@ int pauli_compile(mb_observable o, const mb_term* terms, size_t nterms) {
   o->pauli = pd;
   o->pauli_ok = true;
   for (const OKey& k : o->keys) pd->dense_rows += int64_t(1) << k.k;
-  if (pd->strings.empty()) return MB_OK;
-  std::vector<PFlip> fl;
-  for (const auto& g : pd->groups) fl.push_back(PFlip{g.first, g.second.first, g.second.second});
-  int rc;
-  if ((rc = dev_alloc((void**)&pd->d_flips, sizeof(PFlip) * fl.size())) ||
-      (rc = dev_alloc((void**)&pd->d_all, sizeof(PString) * pd->strings.size()))) {
-    pauli_free(o);
-    return rc;
-  }
-  MB_CHECK_CUDA(cudaMemcpyAsync(pd->d_flips, fl.data(), sizeof(PFlip) * fl.size(), cudaMemcpyHostToDevice, g_ctx.stream));
-  MB_CHECK_CUDA(cudaMemcpyAsync(pd->d_all, pd->strings.data(), sizeof(PString) * pd->strings.size(),
-                                cudaMemcpyHostToDevice, g_ctx.stream));
-  MB_CHECK_CUDA(cudaStreamSynchronize(g_ctx.stream));
   return MB_OK;
 }
 
-bool observable_strings(mb_observable o, int n, ObsStrings* out) {
-  const PauliData* pd = o->pauli;
-  if (!pd) return false;
+// Strings and flip masks on the device, in one buffer, made by the first call that reads them there (45 us
+// of allocations and a wait that an observable of a large pure state never needs). False when they
+// cannot be made now: no room, or a graph is being recorded.
+static bool strings_on_device(PauliData* pd) {
+  if (pd->d_all || pd->strings.empty()) return true;
+  if (g_ctx.capturing) return false;
+  std::vector<PFlip> fl;
+  for (const auto& g : pd->groups) fl.push_back(PFlip{g.first, g.second.first, g.second.second});
+  const size_t at = sizeof(PString) * pd->strings.size(), bytes = at + sizeof(PFlip) * fl.size();
+  std::vector<unsigned char> h(bytes);
+  std::memcpy(h.data(), pd->strings.data(), at);
+  std::memcpy(h.data() + at, fl.data(), bytes - at);
+  void* d = nullptr;
+  if (dev_alloc(&d, bytes)) return false;
+  // pageable source: it has been read when the call returns
+  if (cudaMemcpyAsync(d, h.data(), bytes, cudaMemcpyHostToDevice, g_ctx.stream) != cudaSuccess) {
+    cudaGetLastError();
+    dev_free(d);
+    return false;
+  }
+  pd->d_all = static_cast<PString*>(d);
+  pd->d_flips = reinterpret_cast<PFlip*>(static_cast<unsigned char*>(d) + at);
+  return true;
+}
+
+bool observable_strings(mb_observable o, int n, int64_t most, ObsStrings* out) {
+  PauliData* pd = o->pauli;
+  if (!pd || int64_t(pd->strings.size()) > most) return false;
   for (const auto& g : pd->groups)
     if ((g.first >> n) != 0) return false;
   for (const PString& s : pd->strings)
     if ((s.z >> n) != 0) return false;
+  if (!strings_on_device(pd)) return false;
   *out = ObsStrings{pd->d_flips, pd->d_all, int(pd->groups.size()), int(pd->strings.size())};
   return true;
 }
@@ -463,9 +477,8 @@ bool observable_strings(mb_observable o, int n, ObsStrings* out) {
 // dense keys (MB_EXPECT_KEYS=1 keeps every observable there).
 static bool dm_strings(mb_observable o, int n) {
   if (expect_keys_only()) return false;
-  const PauliData* pd = o->pauli;
   ObsStrings os;
-  return observable_strings(o, n, &os) && os.nstr > 0 && int64_t(os.nstr) <= 4 * pd->dense_rows;
+  return o->pauli && !o->pauli->strings.empty() && observable_strings(o, n, 4 * o->pauli->dense_rows, &os);
 }
 
 int expect_dm_strings(mb_observable o, mb_state s, double2* out, bool* done) {
@@ -501,7 +514,6 @@ int seed_dm_strings(mb_observable o, double2* h, int n, bool* done) {
 
 void pauli_free(mb_observable o) {
   if (!o->pauli) return;
-  dev_free(o->pauli->d_flips);
   dev_free(o->pauli->d_all);
   for (PauliProgram* p : o->pauli->programs) {
     dev_free(p->d_groups);

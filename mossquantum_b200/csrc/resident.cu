@@ -869,7 +869,7 @@ int resident_run(mb_circuit c, mb_observable o, mb_state init, const double* the
   const bool pure = init->kind == MB_PURE || init->kind == MB_BATCH_PURE;
   if (!pure || c->has_channel || n < 1 || n > kResMaxBits || B < 1 || g_ctx.capturing) return MB_OK;
   ObsStrings os;
-  if (!observable_strings(o, n, &os) || os.nstr > 1024) return MB_OK;
+  if (!observable_strings(o, n, 1024, &os)) return MB_OK;
   if (!c->resident) {
     c->resident = new ResidentPlan();
     if (int rc = build_plan(c, c->resident)) {
