@@ -312,6 +312,9 @@ def _matrix_lowering(items):
     return sig, recs, keep
 
 
+_NO_SLOTS = np.zeros(0, dtype=np.intp)
+
+
 class CompiledCircuit:
     """Owner of an ``mb_circuit`` handle."""
 
@@ -376,6 +379,10 @@ class CompiledCircuit:
 
     def _slot_index(self):
         """Parameters that reach the device, and whether they are all of them in order."""
+        if not self.slot_map:
+            self._in_slots = self._slots = _NO_SLOTS
+            self._plain_slots = True
+            return
         self._in_slots = np.array([i for i, s in enumerate(self.slot_map) if s >= 0], dtype=np.intp)
         self._slots = np.array([s for s in self.slot_map if s >= 0], dtype=np.intp)
         self._plain_slots = self._in_slots.size == self.nparams and bool(np.all(self._slots == np.arange(self._slots.size)))
