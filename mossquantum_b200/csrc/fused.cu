@@ -2323,7 +2323,7 @@ static std::string pass_key(const Pass& p, int gen, int R, int N, bool single, i
   return k;
 }
 
-static std::string memo_source(const std::string& key, const std::function<std::string()>& gen) {
+std::string memo_source(const std::string& key, const std::function<std::string()>& gen) {
   static std::mutex mu;
   static std::unordered_map<std::string, std::string> memo;
   static size_t bytes = 0;

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda.h>
 
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -120,6 +121,8 @@ struct PsumPass {
 inline int psum_threads(int t) { return 1 << (t - 4); }
 inline int psum_ctas(int t) { return t >= 12 ? 2 : t == 11 ? 4 : 8; }
 std::string jit_psum_source(const PsumPass& p);
+// Generated source of a key that holds everything its generator reads (fused.cu).
+std::string memo_source(const std::string& key, const std::function<std::string()>& gen);
 int jit_launch_psum(CUfunction fn, const double2* v, const double2* coef, int64_t tps, double2* partials,
                     unsigned* counters, double2* out, int grid, int batch, int t, cudaStream_t st);
 int jit_launch_reg(CUfunction fn, double2* v, const double2* tab, const double2* xtab, const double2* xtabs,

@@ -655,6 +655,32 @@ static int pauli_coefficients(PauliData* pd, PauliProgram* P) {
   return MB_OK;
 }
 
+// Everything jit_psum_source reads: observables that differ in coefficients share their sources.
+static std::string psum_key(const PsumPass& p) {
+  std::string k = "psum";
+  auto put = [&](auto v) { k.append(reinterpret_cast<const char*>(&v), sizeof v); };
+  put(p.n);
+  put(p.t);
+  for (int b : p.bits) put(b);
+  for (const PsumStage& st : p.stages) {
+    for (int r : st.reg) put(r);
+    put(st.groups.size());
+    for (const PsumGroup& g : st.groups) {
+      put(g.xl);
+      put(g.far);
+      put(g.strings.size());
+      for (const PsumString& s : g.strings) {
+        put(s.s);
+        put(s.zr);
+        put(s.zt);
+        put(s.zh);
+        put(char(s.odd | s.re << 1 | s.im << 2));
+      }
+    }
+  }
+  return k;
+}
+
 // Takes the staged passes of a program, compiling them within the limits of every generated kernel (source
 // length, seconds per program) or, without `compile`, only if their kernels are there already. False leaves
 // the program as it was (no placement, no compiler, past a limit, or a kernel that spills).
@@ -663,7 +689,7 @@ static bool pauli_stage(PauliData* pd, PauliProgram* P, bool compile) {
   if (plan.empty()) return false;
   std::vector<std::string> src;
   for (const PsumPass& p : plan) {
-    src.push_back(jit_psum_source(p));
+    src.push_back(memo_source(psum_key(p), [&] { return jit_psum_source(p); }));
     if (src.back().empty() || src.back().size() > jit_max_source()) return false;
   }
   std::vector<CUfunction> fns;
