@@ -452,7 +452,7 @@ struct FOp {
   // diag(1, ph) on bits[0] that may be merged with its neighbours, and a global factor.
   bool merge = false;
   cd ph = cd(1, 0), glob = cd(1, 0);
-  double scale = 1.0;         // MOP_TAN: the factor c left to the pass's MOP_SCALE
+  long double scale = 1.0L;   // MOP_TAN: the factor c left to the pass's MOP_SCALE
 };
 
 // Reverse sweeps: what a gradient is formed from once the passes have run. kind 0: accumulator acc;
@@ -689,14 +689,17 @@ static void mark_unfusable_masks(FOp& f) {
 }
 
 // Rotations with c >= kTanMin run in tangent form, c [[1, -t], [t, 1]] with t = s / c: two
-// multiply-adds per amplitude instead of the shears' three, and a chain of one instead of three. The
-// factors c of a pass are multiplied in once, at its end. The bound keeps an amplitude's growth
-// before that below 2^10 per rotation; beyond it (one in 10^6 of random gates, and gates like Y,
-// whose c is 0) the shears stay. 28 qubits, 20 layers of U3 and CZ: 52.0 ms, 61.4 ms with shears
-// only; a form chosen per gate at run time (a uniform branch) took 57.8 ms.
-constexpr double kTanMin = 1.0 / 1024;
-// Factor product at which a pass multiplies it in before going on (double range: 2^-1022).
-constexpr double kScaleMin = 0x1p-300;
+// multiply-adds per amplitude instead of the shears' three, and a chain of one instead of three, each result
+// rounded once whatever t is. The factors c of a pass are multiplied in after every kScaleEvery rotations
+// and at its end. The generated source must not depend on the matrices' values, or a circuit rebuilt with new
+// angles compiles its passes again, so the bound leaves out exact zeros (gates like Y, which keep the shears)
+// and next to nothing else: angles that round to pi have c = 2^-54. 28 qubits, 20 layers of U3 and CZ:
+// 52.0 ms, 61.4 ms with shears only; a form chosen per gate at run time (a uniform branch) took 57.8 ms.
+constexpr double kTanMin = 0x1p-60;
+// 128 random factors make 2^-92 to 2^-128. A product that passes kScaleMin all the same (some fifty angles
+// within 1e-3 of pi) is multiplied in before the pass goes on; amplitudes up to 2^363 stay in range.
+constexpr int kScaleEvery = 128;
+constexpr double kScaleMin = 0x1p-600;
 
 // A fixed 2x2 as E = g * diag(1, A) * R * diag(1, B), R = [[c, -s], [s, c]] with c = |e00| and
 // s = |e10|, so that R runs as three shears with t = s / (1 + c) <= 1. Returns false (the gate
@@ -836,8 +839,14 @@ static bool split_fixed_1q(mb_circuit circ, const FOp& f, bool dm, std::vector<d
   r.tgt[0] = q;
   r.ntgt = 1;
   r.cls = CLS_DENSE;
-  r.scale = r.type == MOP_TAN ? c : 1.0;
-  r.off[0] = xtab_push(xt, r.type == MOP_TAN ? make_double2(sn / c, c) : make_double2(mt, sn));
+  if (r.type == MOP_TAN) {
+    // the rounding of t stays in the smaller of the two entries: c t = s where s is the larger
+    const double t = sn / c;
+    r.scale = t > 1.0 ? (long double)sn / t : (long double)c;
+    r.off[0] = xtab_push(xt, make_double2(t, double(r.scale)));
+  } else {
+    r.off[0] = xtab_push(xt, make_double2(mt, sn));
+  }
   finalize_masks(r);
   seq.push_back(r);
   FOp pa;
@@ -1385,12 +1394,22 @@ static bool tile_geom(const std::vector<int>& bits, int N, int nsamples, TmaGeom
   return true;
 }
 
-static MOp scale_mop(double scale, std::vector<double2>* xt) {
-  MOp m{};
-  m.type = MOP_SCALE;
-  m.off[0] = xtab_push(xt, make_double2(scale, 0.0));
-  return m;
-}
+// Factors of a pass's tangent rotations that are not multiplied in yet.
+struct Gathered {
+  long double scale = 1.0L;
+  int count = 0;
+  void add(const FOp& f) {
+    if (f.type == MOP_TAN) scale *= f.scale, ++count;
+  }
+  bool due() const { return count == kScaleEvery || scale < kScaleMin; }
+  MOp take(std::vector<double2>* xt) {
+    MOp m{};
+    m.type = MOP_SCALE;
+    m.off[0] = xtab_push(xt, make_double2(double(scale), 0.0));
+    *this = Gathered();
+    return m;
+  }
+};
 
 // Register stages of a tile pass: every stage loads 2^R amplitudes per thread over R
 // tile-local bits and applies the ops whose targets lie among them.
@@ -1428,7 +1447,7 @@ static void plan_stages(const std::vector<FOp>& fops, const std::vector<int>& op
   uint64_t wmask = 0;
   for (int q : wbits) wmask |= uint64_t(1) << q;
   std::vector<int> rem = ops;
-  double scale = 1.0;   // factors of the pass's tangent rotations not multiplied in yet
+  Gathered gathered;
   while (!rem.empty()) {
     std::vector<int> regs;
     uint64_t rmask = 0, b_all = 0, b_nd = 0;
@@ -1652,19 +1671,18 @@ static void plan_stages(const std::vector<FOp>& fops, const std::vector<int>& op
       emit(fops[taken[i]]);
       p.fop_order.push_back(taken[i]);
       ++nemit;
-      scale *= fops[taken[i]].scale;
-      if (scale < kScaleMin) {
-        p.mops.push_back(scale_mop(scale, xt));
+      gathered.add(fops[taken[i]]);
+      if (gathered.due()) {
+        p.mops.push_back(gathered.take(xt));
         ++nemit;
-        scale = 1.0;
       }
     }
     sd.nops = nemit;
     p.stages.push_back(sd);
     rem.swap(left);
   }
-  if (scale != 1.0 && !p.stages.empty()) {
-    p.mops.push_back(scale_mop(scale, xt));
+  if (gathered.count && !p.stages.empty()) {
+    p.mops.push_back(gathered.take(xt));
     p.stages.back().nops += 1;
   }
 }
@@ -1676,7 +1694,7 @@ static void encode_reg_pass(const std::vector<FOp>& fops, const std::vector<int>
   sd.nreg = R;
   for (int k = 0; k < R; ++k) sd.reg[k] = p.bits[k];
   sd.op0 = 0;
-  double scale = 1.0;
+  Gathered gathered;
   for (int idx : ops) {
     const FOp& f = fops[idx];
     p.fop_order.push_back(idx);
@@ -1719,13 +1737,10 @@ static void encode_reg_pass(const std::vector<FOp>& fops, const std::vector<int>
       for (int j = 0; j < f.nctrl; ++j) m.sel[j] = int16_t(f.ctrl[j]);
     }
     p.mops.push_back(m);
-    scale *= f.scale;
-    if (scale < kScaleMin) {
-      p.mops.push_back(scale_mop(scale, xt));
-      scale = 1.0;
-    }
+    gathered.add(f);
+    if (gathered.due()) p.mops.push_back(gathered.take(xt));
   }
-  if (scale != 1.0) p.mops.push_back(scale_mop(scale, xt));
+  if (gathered.count) p.mops.push_back(gathered.take(xt));
   sd.nops = int(p.mops.size());
   p.stages.push_back(sd);
 }
