@@ -3147,7 +3147,7 @@ extern "C" int mb_schedule_info(const mb_op* ops, size_t nops, int n, int dm, in
         int j = 0;
         for (mb::Pass& ps : A.passes) {
           if (ps.kind != mb::PASS_TILE) continue;
-          const std::string src = mb::jit_adjoint_source(ps, A.R, N, nsamples == 1, mb::adjoint_ctas(ps.t, A.dm));
+          const std::string src = mb::jit_adjoint_source(ps, A.R, N, true, mb::adjoint_ctas(ps.t, A.dm));
           char path[512];
           snprintf(path, sizeof(path), "%s/adj_%03d.cu", dir, j++);
           if (FILE* f = fopen(path, "w")) {
