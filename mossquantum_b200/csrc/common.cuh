@@ -97,6 +97,8 @@ struct ProfScope {
   ProfScope(const char* name, double bytes, cudaStream_t stream, double flops = 0);
   ~ProfScope();
 };
+// Counts a launch under a second name, without a time of its own.
+void prof_count(const char* name);
 
 inline int grid_for(int64_t work, int block, int64_t cap = int64_t(148) * 32) {
   int64_t g = (work + block - 1) / block;

@@ -967,6 +967,7 @@ int expect_pauli(mb_observable o, mb_state s, double2* out) {
       if (int rc = jit_launch_psum((CUfunction)f, s->d, P->d_coef, tps, g_ctx.partials, g_ctx.counters, out, G, s->batch,
                                    P->psum_t, st))
         return rc;
+      prof_count("mbk_psum");
       MB_LAUNCHED();
     }
     return MB_OK;

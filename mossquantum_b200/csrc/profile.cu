@@ -65,6 +65,10 @@ ProfScope::~ProfScope() {
   if (slot >= 0 && slot < int(g_pending.size())) cudaEventRecord(g_pending[slot].b, st);
 }
 
+void prof_count(const char* name) {
+  if (g_prof) g_stats[name].launches += 1;
+}
+
 }  // namespace mb
 
 using namespace mb;
