@@ -180,7 +180,8 @@ __device__ __forceinline__ CDD lane_of(const CDD& v, int src) {
 // dependent reads (offset, entry), so four components are read together: 40 records of up to 16
 // components (density matrix of 10 qubits) took 45 us with one thread per record, now 21. All lanes of
 // the warp enter (a lane without a record passes nc = 0): groups run to the longest record of the warp.
-// 2x2 products are kept in double-double and rounded once: a product's error acts alike on every
+// 2x2 products are kept in double-double and rounded once (4x4 products, and those of fixed gates formed on the
+// host, are rounded gate by gate): a product's error acts alike on every
 // amplitude of a state (gradients of 20 and 22 qubits, 16 sets of angles, largest error relative to the
 // largest entry: mean 1.6e-15 and 1.5e-15, 2.2e-15 rounded gate by gate; 12.6 against 11.3 us per launch).
 template <int G>
@@ -2056,9 +2057,9 @@ static Tuning tuning_for(int N, bool whole = true) {
     // 2^10-amplitude tiles. The passes load the FP64 pipe and the shared-memory pipe alike (55 to
     // 60 % of each), so 16 amplitudes per thread with 6 CTAs of 64 threads beat 8 amplitudes with 4
     // CTAs of 128: fewer stages move the tile, half the warps read the matrices. 28-qubit U3 + CZ
-    // step 48.5 against 51.4 ms, 20 x 20 RX/RY/RZ + CNOT 405 against 425 us, noisy 11 qubits 562
-    // against 610. Below 2^20 amplitudes 64-thread CTAs leave the chip short of warps (18 qubits: 137
-    // against 122 us, noisy 9 qubits 102 against 96), and the short segments of a checkpointed
+    // step 48.7 against 52.0 ms, 20 x 20 RX/RY/RZ + CNOT 388 against 415 us a call, noisy 11 qubits 616
+    // against 663. Below 2^20 amplitudes 64-thread CTAs leave the chip short of warps (18 qubits: 140.5
+    // against 138 us a call, noisy 9 qubits 145 against 142), and the short segments of a checkpointed
     // gradient are mostly light passes (24 qubits: 6.50 against 6.36 ms). 32 amplitudes with
     // 6 warps: no faster, compile times past the budget. 2^11 tiles: 5.62 against 5.43 ms (25 qubits).
     tu.t = 10;

@@ -1,4 +1,4 @@
-// Bind-time fusion of consecutive operations on one qubit (host and device).
+// Bind-time fusion of consecutive operations on one qubit.
 //
 // A run of operations that act only on qubit q (pure states: bit q; density matrices: the row
 // bit q and the column bit q + n) multiplies into one 2x2 (pure) or 4x4 (density) matrix. For
@@ -36,9 +36,10 @@ struct FuseRec {
   int32_t c0, nc; // components [c0, c0 + nc) in application order
 };
 
-// M (d x d, column-major) = product of the record's components, the last one leftmost.
-__host__ __device__ inline void fuse_product(const FuseRec& r, const FuseComp* comps, const double2* row0,
-                                             const double2* rowb, double2* M) {
+// M (d x d, column-major) = product of the record's components, the last one leftmost; on the host, each
+// component's product rounded as it is formed (k_fuse's 4x4 products likewise; its 2x2 ones once).
+inline void fuse_product(const FuseRec& r, const FuseComp* comps, const double2* row0,
+                         const double2* rowb, double2* M) {
   const int d = r.d;
   for (int i = 0; i < d * d; ++i) M[i] = make_double2((i % (d + 1)) == 0 ? 1.0 : 0.0, 0.0);
   for (int ci = 0; ci < r.nc; ++ci) {
@@ -88,7 +89,8 @@ __host__ __device__ inline void fuse_product(const FuseRec& r, const FuseComp* c
   }
 }
 
-// A run's product is rounded once: its entries are carried as high and low parts, because an error
+// A parametric 2x2 run's product is rounded once: its entries are carried as high and low parts (Knuth's
+// two-sum, and the error of a product by one fused multiply-add), because an error
 // of the matrix is the same for every amplitude and adds up over the steps, where roundings of
 // amplitudes average out.
 struct DD {

@@ -1524,7 +1524,8 @@ std::string jit_pauli_source(const PauliJitPass& p, int max_vals) {
 // higher index bits into the low three, so eight lanes whose bits differ mod 3 never conflict.
 // Bound: reading the state once per pass (2^26 amplitudes: 166 us), then shared-memory reads (16 B per
 // amplitude and stage). XXZ on 26 qubits: 3 passes, 618 us in all, against 4.6 ms for 4 interpreted
-// passes that read a partner from the tile per group and evaluated signs per amplitude.
+// passes that read a partner from the tile per group and evaluated signs per amplitude; error over 16 random
+// states of norm 1: mean 1.9e-17, largest 6.9e-17 (2.8e-17 and 6.0e-17 interpreted).
 std::string jit_psum_source(const PsumPass& p) {
   const int t = p.t, T = psum_threads(t), A = 16;
   std::ostringstream body;
