@@ -941,7 +941,8 @@ extern "C" int mb_apply(mb_circuit c, mb_state s, const double* theta, size_t nt
     return MB_EINVAL;
   }
   const int rows = per_sample ? s->batch : 1;
-  if (rows == 0) return MB_OK;
+  // An empty batch has nothing to apply to, and its schedule no row for the products of fused runs.
+  if (s->batch == 0) return per_sample || (flags & MB_APPLY_DEVICE_THETA) ? MB_OK : theta_check(c, theta, ntheta, rows);
   if (flags & MB_APPLY_DEVICE_THETA) {
     if (c->theta_rows != rows) {
       set_error("mb_apply: staged parameters have %d rows, the state needs %d", c->theta_rows, rows);
@@ -1214,6 +1215,7 @@ extern "C" int mb_observable_apply(mb_observable o, mb_state in, mb_state out) {
     return MB_EINVAL;
   }
   if (int rc = validate_observable(o, in)) return rc;
+  if (in->batch == 0) return MB_OK;
   const int is_dm = in->kind == MB_DENSITY || in->kind == MB_BATCH_DENSITY;
   if (!is_dm && o->pauli_ok && !g_ctx.capturing) {
     // pure states from 10 qubits: Pauli-string passes over shared-memory tiles
