@@ -229,11 +229,12 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
   }
   const char* plain_env = getenv("MB_ADJOINT_PLAIN");
   const bool plain_only = plain_env && atoi(plain_env);
-  if (!is_dm && !plain_only) {
+  const bool unitary = circuit_unitary(c);
+  if (!is_dm && !plain_only && unitary) {
     // small pure states: values and gradient in one launch
     bool done = false;
     std::vector<double2> v(B);
-    if ((rc = resident_run(c, o, init, theta, w.data(), checkpoint_every, v.data(), grad, &done))) return rc;
+    if ((rc = resident_run(c, o, init, theta, w.data(), v.data(), grad, &done))) return rc;
     if (done) {
       double total = 0;
       for (int b = 0; b < B; ++b) total += w[b] * v[b].x;
@@ -246,6 +247,8 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
   // parameters, so on density matrices (batches, and pure batches promoted by a channel) the
   // weighted sum of the samples goes through the circuit once in their place.
   const bool combine = is_dm && B > 1;
+  bool uniform_w = true;
+  for (int b = 1; b < B; ++b) uniform_w = uniform_w && w[b] == w[0];
   const size_t sbytes = sizeof(double2) * size_t(elems) * (combine ? 1 : B);
   Buf d_w, d_grad, y, delta;
   if ((rc = d_w.alloc(sizeof(double) * B)) || (rc = d_grad.alloc(sizeof(double) * std::max(1, c->nslots))) ||
@@ -267,7 +270,7 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
 
   // Fused path: pure states with unitary circuits (specialised dual-state passes).
   const int nops_all = int(c->ops.size());
-  if (!is_dm && !c->has_channel && n >= 9 && nops_all > 0 && !plain_only) {
+  if (!is_dm && !c->has_channel && n >= 9 && nops_all > 0 && !plain_only && (B == 1 || unitary)) {
     const int kf = checkpoint_every > 0 ? checkpoint_every : nops_all;
     const int Sf = (nops_all + kf - 1) / kf;
     std::vector<Schedule*> adj(Sf, nullptr), fwd(Sf, nullptr);
@@ -325,7 +328,7 @@ extern "C" int mb_adjoint(mb_circuit c, mb_observable o, mb_state init, const do
   // inverses. Segments end at checkpoint_every and wherever the product of the channels'
   // ||S^-1||_2 would pass 100, so the rounding error of the uncomputed y stays bounded; y is
   // reset to the segment's checkpoint after each reversed segment.
-  if (is_dm && 2 * n >= 8 && nops_all > 0 && !plain_only) {
+  if (is_dm && 2 * n >= 8 && nops_all > 0 && !plain_only && (uniform_w || unitary)) {
     std::vector<int> cuts = {0};
     bool ok = true;
     double growth = 1.0;

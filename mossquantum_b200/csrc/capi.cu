@@ -720,6 +720,25 @@ int check_not_capturing(const char* what) {
   return MB_OK;
 }
 
+bool circuit_unitary(mb_circuit c) {
+  if (c->unitary >= 0) return c->unitary != 0;
+  c->unitary = 1;
+  for (const COp& op : c->ops) {
+    if (op.kind != MB_OP_GATE || op.parametric) continue;
+    const double2* M = c->fixed_table.data() + op.mat_off;
+    const int d = 1 << op.k;
+    for (int a = 0; a < d && c->unitary; ++a)
+      for (int b = 0; b < d; ++b) {
+        double2 x = make_double2(a == b ? -1.0 : 0.0, 0.0);   // (U'U - 1)[a, b]
+        for (int r = 0; r < d; ++r) x = cfma_conj(M[r + d * a], M[r + d * b], x);
+        // the rounding of a matrix formed in double precision
+        if (!(std::fabs(x.x) <= 1e-12 && std::fabs(x.y) <= 1e-12)) c->unitary = 0;
+      }
+    if (!c->unitary) break;
+  }
+  return c->unitary != 0;
+}
+
 int theta_check(mb_circuit c, const double* theta, size_t ntheta, int rows) {
   if (ntheta != size_t(c->nslots) * rows) {
     set_error("expected %zu parameter values, got %zu", size_t(c->nslots) * rows, ntheta);
@@ -1157,7 +1176,7 @@ extern "C" int mb_objective_values(mb_circuit c, mb_observable o, mb_state init,
   }
   if (!expect_keys_only()) {
     bool done = false;
-    if (int rc = resident_run(c, o, init, theta, nullptr, 0, reinterpret_cast<double2*>(out), nullptr, &done)) return rc;
+    if (int rc = resident_run(c, o, init, theta, nullptr, reinterpret_cast<double2*>(out), nullptr, &done)) return rc;
     if (done) return MB_OK;
   }
   // The general form: a private copy of the initial state through the fused passes.

@@ -1248,7 +1248,7 @@ static bool build_adjoint_fops(mb_circuit c, int lo, int hi, std::vector<FOp>& o
     }
     if (op.gen_off >= 0) seq.back().grad = oi;   // density matrices: once both halves are undone
   }
-  if (!dm && !getenv("MB_NO_FUSE")) fuse_runs(c, seq, n, false, S);
+  if (!dm && circuit_unitary(c) && !getenv("MB_NO_FUSE")) fuse_runs(c, seq, n, false, S);
   auto gradient = [&](const COp& op, int shift) {
     FOp g = grad_fop(op, shift);
     S->accs.push_back(AccRec{0, S->nacc, op.slot, 0, 0, 0});

@@ -58,6 +58,7 @@ struct mb_circuit_s {
   int theta_rows = 0;                 // rows staged by the last theta upload
   std::vector<mb::Schedule*> scheds;  // fused schedules, built lazily per state shape
   mb::ResidentPlan* resident = nullptr;  // built lazily by the first small objective
+  int unitary = -1;                      // circuit_unitary, once asked
 };
 
 namespace mb {
@@ -158,6 +159,9 @@ struct SmallBufs {
 // Target local bit of a fixed matrix that is the identity unless every other bit is 1, or -1.
 int controlled_target(const double2* M, int k);
 int check_not_capturing(const char* what);
+// Whether every fixed gate matrix is unitary. Reverse sweeps undo gates by their adjoints, so only then may gates on
+// different qubits change places, and only then are checkpoints a matter of rounding.
+bool circuit_unitary(mb_circuit c);
 int plain_op(mb_circuit c, const COp& op, double2* v, int n, int is_dm, int nsamples, int64_t mrow_stride,
              bool dagger);
 int circuit_clone(mb_circuit src, mb_circuit* out);
@@ -195,11 +199,10 @@ int reverse_dm_single(mb_circuit c, int n, const double2* ckpt, double2* delta, 
                       double2* const* scratch);
 
 // resident.cu: small pure states, the whole objective in one launch. values: <H> per sample;
-// grad (or null): the gradient of the weighted sum. *done = false when the circuit, the
-// observable or the size has no resident form, or checkpoints (checkpoint_every > 0) would change
-// the gradient (nothing has been launched then).
+// grad (or null): the gradient of the weighted sum (unitary circuits only). *done = false when the
+// circuit, the observable or the size has no resident form (nothing has been launched then).
 int resident_run(mb_circuit c, mb_observable o, mb_state init, const double* theta, const double* weights,
-                 int checkpoint_every, double2* values, double* grad, bool* done);
+                 double2* values, double* grad, bool* done);
 void resident_release(mb_circuit c);
 
 // pauli.cu

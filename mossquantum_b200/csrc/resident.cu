@@ -89,7 +89,6 @@ struct ResidentPlan {
   int n = 0;
   bool ok = false;
   bool unique = true;               // every slot has one gate
-  bool unitary = true;              // every fixed matrix is
   int nstages = 0, ngroups = 0, nops = 0, ncs = 0, nmat = 0, ngrad = 0;   // ngrad: groups with gradients
   uint16_t row[kResMaxBits] = {0}, col[kResMaxBits] = {0}, rconst = 0;  // frame after the circuit
   void* d = nullptr;                // stages, groups, ops, angles, matrix offsets
@@ -669,16 +668,6 @@ struct Builder {
     open[t].push_back(Held{op, controls(ctl, nctl)});
     if (nctl) close(t);
   }
-  // U'U = 1 up to the rounding of a matrix formed in double precision.
-  static bool unitary(const double2* M, int d) {
-    for (int a = 0; a < d; ++a)
-      for (int b = 0; b < d; ++b) {
-        double2 x = make_double2(a == b ? -1.0 : 0.0, 0.0);
-        for (int r = 0; r < d; ++r) x = cfma_conj(M[r + d * a], M[r + d * b], x);
-        if (!(std::fabs(x.x) <= 1e-12 && std::fabs(x.y) <= 1e-12)) return false;
-      }
-    return true;
-  }
   uint16_t matrix(const COp& o, int count, const int* elems) {
     const uint16_t at = uint16_t(mats.size());
     for (int e = 0; e < count; ++e) mats.push_back(o.mat_off + elems[e]);
@@ -713,7 +702,6 @@ struct Builder {
       return true;
     }
     const double2* M = c->fixed_table.data() + o.mat_off;
-    P->unitary = P->unitary && unitary(M, d);
     auto is = [&](int r, int cc, double x) { return M[r + d * cc].x == x && M[r + d * cc].y == 0.0; };
     // SWAP
     if (o.k == 2 && is(0, 0, 1) && is(1, 2, 1) && is(2, 1, 1) && is(3, 3, 1) && o.cls == CLS_MONO) {
@@ -864,7 +852,7 @@ void resident_release(mb_circuit c) {
 }
 
 int resident_run(mb_circuit c, mb_observable o, mb_state init, const double* theta, const double* weights,
-                 int checkpoint_every, double2* values, double* grad, bool* done) {
+                 double2* values, double* grad, bool* done) {
   *done = false;
   const int n = c->n, B = init->batch;
   const bool pure = init->kind == MB_PURE || init->kind == MB_BATCH_PURE;
@@ -882,9 +870,6 @@ int resident_run(mb_circuit c, mb_observable o, mb_state init, const double* the
   }
   const ResidentPlan& P = *c->resident;
   if (!P.ok) return MB_OK;
-  // The reverse undoes every gate by its adjoint. Checkpoints differ from that by rounding while the
-  // matrices are unitary; otherwise a sweep with checkpoints reads the states back that this one cannot.
-  if (grad && checkpoint_every > 0 && !P.unitary) return MB_OK;
   const int T = resident_threads(n);
   // Rows per chunk: 32 KiB of partial cross sums.
   const int chunk = std::max(4, 4096 / T);
