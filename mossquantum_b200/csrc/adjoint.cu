@@ -11,7 +11,9 @@
 // Circuits with channels run on density matrices throughout (a pure initial state is
 // promoted first, DensityMatrix(psi), execution/channels.jl:19); this gives the same
 // parameter gradient as promoting at the first channel.
-// Batches of density matrices enter as their weighted sum (the loss is linear in them).
+// Batches of density matrices enter as their weighted sum (the loss is linear in them). The adjoint of a
+// matrix that is not unitary does not undo it, so the order of the gates matters then (circuit_unitary): pure batches
+// and density matrices with unequal weights go gate by gate.
 // Fused paths: pure states and density matrices run the reverse as dual-state passes (y and Δ tiles together, gradients accumulated in the
 // pass). On density matrices a single-qubit channel is reversed by S' on Δ and S^-1 on y (the
 // input is uncomputed instead of recomputed); segments keep the product of ||S^-1||_2 within
